@@ -1,4 +1,4 @@
-// Batched complex GEMM problems: D = alpha * op(A) op(B) + beta * Csrc.
+// Batched complex GEMM problems: D = alpha * op(A) op(B) + beta * Csrc + eye * I.
 // Each batch entry is a GemmProb in device memory, so kernels that build the
 // problems on the device (from gate descriptors) and the host API share one
 // launcher.  op: 0 = N, 1 = T, 2 = C (conjugate transpose).
@@ -14,6 +14,7 @@ struct GemmProb {
   int M, N, K;
   int opA, opB;
   double alpha_re, alpha_im, beta_re, beta_im;
+  double eye;  // added to the diagonal of D
 };
 
 // Optional tensor-core context: the tensor-core path's scratch token and a

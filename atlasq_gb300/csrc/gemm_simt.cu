@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
       if (c >= p.N) continue;
       CX v = cmul(alpha, acc[i][j]);
       if (use_beta) v = cadd(v, cmul(beta, C[(int64_t)r * p.ldc + c]));
+      if (r == c) v.x += (R)p.eye;
       D[(int64_t)r * p.ldd + c] = v;
     }
   }
@@ -156,6 +157,7 @@ extern "C" int agb_cgemm_batched(int dtype, char opA, char opB, int batch, int M
   b.alpha_im = alpha_im;
   b.beta_re = beta_re;
   b.beta_im = beta_im;
+  b.eye = 0;
   sb.sA = strideA;
   sb.sB = strideB;
   sb.sC = strideC;

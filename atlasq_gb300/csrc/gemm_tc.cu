@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     float2* D = (float2*)P.D;
     const float2* C = (const float2*)P.Csrc;
     const float ar = (float)P.alpha_re, ai = (float)P.alpha_im, br = (float)P.beta_re, bi = (float)P.beta_im;
+    const float eye = (float)P.eye;
     const bool use_beta = (br != 0.f || bi != 0.f);
     const int nacc = nk < NACC ? nk : NACC;
 #pragma unroll 1
@@ -381,6 +382,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               v.x += br * c.x - bi * c.y;
               v.y += br * c.y + bi * c.x;
             }
+            if (row == col) v.x += eye;
             D[(int64_t)row * P.ldd + col] = v;
           }
         }
@@ -489,6 +491,7 @@ static int cgemm_tc_impl(char opA, char opB, int batch, int M, int N, int K, con
   base.alpha_im = alpha_im;
   base.beta_re = beta_re;
   base.beta_im = beta_im;
+  base.eye = 0;
   char* w = (char*)ws;
   GemmProb* probs = (GemmProb*)w;
   int* status = (int*)(w + agb_align((size_t)batch * sizeof(GemmProb)));

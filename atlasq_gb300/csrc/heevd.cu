@@ -1000,7 +1000,10 @@ __global__ void __launch_bounds__(256) cluster_invit_kernel(const HeevdProb* __r
 
 // ------------------------------------------------------------------ stage 5 (backtransform2_kernel below)
 // ------------------------------------------------------------------ stage 6
-// GEMM problems for one Newton-Schulz step: M = Vs^H Vs; Vd = 1.5 Vs - 0.5 Vs M
+// GEMM problems for one Newton-Schulz step, in its residual form:
+// M = I - Vs^H Vs; Vd = Vs + 0.5 Vs M.  The product with Vs is then a small
+// correction, whose rounding does not reach Vd (the form 1.5 Vs - 0.5 Vs (Vs^H Vs)
+// carries the rounding of a product of the size of Vs).
 __global__ void polish_setup_kernel(HeevdProb* __restrict__ probs, GemmProb* gp, int count,
                                     int step) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1023,7 +1026,7 @@ __global__ void polish_setup_kernel(HeevdProb* __restrict__ probs, GemmProb* gp,
   g.lda = lds; g.ldb = lds; g.ldd = P.ell; g.ldc = P.ell;
   g.M = P.nvec; g.N = P.nvec; g.K = P.n;
   g.opA = 2; g.opB = 0;
-  g.alpha_re = 1; g.alpha_im = 0; g.beta_re = 0; g.beta_im = 0;
+  g.alpha_re = -1; g.alpha_im = 0; g.beta_re = 0; g.beta_im = 0; g.eye = 1;
   if (idle) g.M = 0;
   gp[i] = g;
   GemmProb h;
@@ -1031,12 +1034,12 @@ __global__ void polish_setup_kernel(HeevdProb* __restrict__ probs, GemmProb* gp,
   h.lda = lds; h.ldb = P.ell; h.ldd = ldd; h.ldc = lds;
   h.M = P.n; h.N = P.nvec; h.K = P.nvec;
   h.opA = 0; h.opB = 0;
-  h.alpha_re = -0.5; h.alpha_im = 0; h.beta_re = 1.5; h.beta_im = 0;
+  h.alpha_re = 0.5; h.alpha_im = 0; h.beta_re = 1; h.beta_im = 0; h.eye = 0;
   if (idle) h.M = 0;
   gp[count + i] = h;
 }
 
-// Orthogonality guard on the first polish product M = V^H V (row stride ell).
+// Orthogonality guard on the first polish product M = I - V^H V (row stride ell).
 // Only eigenvectors whose eigenvalue lies above the float rounding level of
 // the Gram matrix (64 ulp of lambda_0, the level below which the rank rule
 // cannot see a value) are checked: vectors of numerically-zero eigenvalues

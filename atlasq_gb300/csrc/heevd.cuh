@@ -139,6 +139,13 @@ int tridiag_cluster_size(int esz, int n);
 template <typename CX>
 int launch_tridiag_cluster(const HeevdProb* probs, int count, int maxn, cudaStream_t s);
 
+// Register-resident form (complex64), tridiag_reg.cu: the clusters of C CTAs the
+// device holds at once, the CTAs per matrix it chooses for a batch, and its
+// launch with C of them.
+int tridiag_reg_clusters(int maxn, int C);
+int tridiag_reg_ctas(int maxn, int count);
+int launch_tridiag_reg(const HeevdProb* probs, int count, int maxn, int C, cudaStream_t s);
+
 // Launch all stages.  `probs` is a device array of `count` problems with
 // n <= maxn and ell <= maxell; `gemm_scratch` holds 4*count GemmProb entries.
 template <typename CX>

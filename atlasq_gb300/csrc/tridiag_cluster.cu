@@ -1,5 +1,6 @@
-// Householder tridiagonalisation of a Hermitian matrix held in the distributed
-// shared memory of a thread-block cluster (sm_103a).
+// Householder tridiagonalisation of a complex128 Hermitian matrix held in the
+// distributed shared memory of a thread-block cluster (sm_103a), and the
+// cluster-size choice for both types (complex64 runs in tridiag_reg.cu).
 //
 // One cluster of C CTAs (C = 1, 2, 4 or 8) per matrix.  CTA q owns the rows
 // r = q, q + C, q + 2C, ... and keeps their lower-triangular entries packed in
@@ -17,7 +18,7 @@
 // Outputs match the single-CTA kernel: d, e (real), tau (complex), reflector v_j
 // in row j of H (columns j+2 .. n-1, v_j[j+1] = 1 implicit), scale.
 //
-// Rows that do not fit (matrices above ~700 for complex64 at 8 CTAs) stay in
+// Rows that do not fit (matrices above ~460 at 8 CTAs) stay in
 // place in the lower triangle of H (L2-resident): a CTA keeps its first
 // `isplit` rows (the short ones) in shared memory and addresses the rest as
 // H[r][0..r].  The reflectors are written to the strictly upper part of H
@@ -283,19 +284,15 @@ size_t tridiag_cluster_smem(int esz, int n, int C) {
 namespace {
 constexpr size_t kSmemBudget = 224 * 1024;
 
-// Largest cluster the device can co-schedule with `smem` bytes per CTA (16 needs
-// the non-portable opt-in); 0 if none.
-template <typename CX>
-int max_cluster(size_t smem) {
-  static int cached[2][2] = {{-1, -1}, {-1, -1}};
-  const int big = smem > 160 * 1024;
-  int& c = cached[sizeof(CX) == 16][big];
+// Largest cluster the device can co-schedule with the full shared-memory budget
+// per CTA (16 needs the non-portable opt-in).
+int max_cluster() {
+  static int c = -1;
   if (c >= 0) return c;
   c = 8;
-  if (cudaFuncSetAttribute(tridiag_cluster_kernel<CX, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-      cudaSuccess) {
-    cudaFuncSetAttribute(tridiag_cluster_kernel<CX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemBudget);
+  const auto kern = tridiag_cluster_kernel<double2, true>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(16, 1, 1);
     cfg.blockDim = dim3(512, 1, 1);
@@ -308,9 +305,7 @@ int max_cluster(size_t smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, tridiag_cluster_kernel<CX, true>, &cfg) == cudaSuccess &&
-        nclusters > 0)
-      c = 16;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters > 0) c = 16;
   }
   cudaGetLastError();
   return c;
@@ -324,27 +319,31 @@ static int g_tuned_T[2][33][3] = {};  // threads per CTA (256 or 512), 0 = 512
 static int count_class(int count) { return count <= 8 ? 0 : (count <= 32 ? 1 : 2); }
 
 static bool cluster_fits(int esz, int n, int C) {
+  if (esz == 8) return tridiag_reg_clusters(n, C) > 0;
   if (C <= 8) return tridiag_cluster_smem(esz, n, C) <= kSmemBudget || C == 8;
   return 6 * (size_t)n * esz + 64 * 1024 <= kSmemBudget;
 }
 
 // Pick the cluster size for a matrix of size n: the autotuned choice for this
-// size and batch class if there is one; otherwise the smallest of 1..8 CTAs
-// whose shared memory holds every row (at least 8 above n = 256, where the
-// per-step work, not the barriers, dominates); else the largest cluster the
-// device schedules, with the overflow rows in L2.
+// size and batch class if there is one; otherwise for complex64 the register
+// form's own rule, for complex128 the smallest of 1..8 CTAs whose shared memory
+// holds every row (at least 8 above n = 256, where the per-step work, not the
+// barriers, dominates); else the largest cluster the device schedules, with
+// the overflow rows in L2.
 int tridiag_cluster_size_for(int esz, int n, int count) {
   const int t = g_tuned_C[esz == 16][(n + 31) / 32][count_class(count)];
   if (t > 0 && cluster_fits(esz, n, t)) return t;
+  if (esz == 8) return tridiag_reg_ctas(n, count);
   return tridiag_cluster_size(esz, n);
 }
 
 int tridiag_cluster_size(int esz, int n) {
+  if (esz == 8) return tridiag_reg_ctas(n, 1);
   const int lo = n > 256 ? 8 : 1;
   for (int C = lo; C <= 8; ++C)
     if (tridiag_cluster_smem(esz, n, C) <= kSmemBudget) return C;
   if (6 * (size_t)n * esz + 64 * 1024 > kSmemBudget) return 0;
-  return esz == 8 ? max_cluster<float2>(kSmemBudget) : max_cluster<double2>(kSmemBudget);
+  return max_cluster();
 }
 
 template <typename CX>
@@ -363,6 +362,10 @@ template <typename CX>
 int launch_tridiag_cluster_C(const HeevdProb* probs, int count, int maxn, int C, cudaStream_t s, int threads) {
   const int esz = sizeof(CX);
   if (C == 0) return AGB_ERR_UNSUPPORTED;
+  if constexpr (sizeof(CX) == 8) {
+    (void)threads;  // its CTAs have one size
+    return launch_tridiag_reg(probs, count, maxn, C, s);
+  } else {
   size_t smem = tridiag_cluster_smem(esz, maxn, C);
   const bool overflow = smem > kSmemBudget;
   if (overflow) smem = kSmemBudget;
@@ -389,6 +392,7 @@ int launch_tridiag_cluster_C(const HeevdProb* probs, int count, int maxn, int C,
     return AGB_ERR_CUDA;
   }
   return AGB_OK;
+  }
 }
 
 template int launch_tridiag_cluster<float2>(const HeevdProb*, int, int, cudaStream_t);
@@ -448,6 +452,7 @@ int tune_impl(int n, int count, void* ws, size_t ws_bytes, cudaStream_t s, int* 
   float bms = 1e30f;
   for (int k = 0; k < 2 * nc; ++k) {
     const int thr = (k & 1) ? 256 : 512;
+    if (esz == 8 && thr == 256) continue;  // one CTA size
     float tot = 0;
     for (int rep = 0; rep < 3; ++rep) {
       tune_fill_kernel<CX><<<dim3(64, count), 256, 0, s>>>(probs, base, count, n, stride, esz, 1234 + rep);
@@ -509,11 +514,8 @@ extern "C" int agb_set_tridiag_cluster(int dtype, int n, int count, int C, int t
   if (n <= 0 || n > 1024 || count <= 0 || C < 0 || C > 16 || (threads != 256 && threads != 512)) return AGB_ERR_ARG;
   const int esz = dtype == AGB_C64 ? 8 : 16;
   if (C > 0 && (C > n || !cluster_fits(esz, n, C))) return AGB_ERR_UNSUPPORTED;
-  if (C > tridiag_cluster_size(esz, n) && C > 8) {
-    // a non-portable size must be one the device schedules
-    const int maxC = esz == 8 ? max_cluster<float2>(kSmemBudget) : max_cluster<double2>(kSmemBudget);
-    if (C > maxC) return AGB_ERR_UNSUPPORTED;
-  }
+  // a non-portable size must be one the device schedules (complex64: cluster_fits)
+  if (esz == 16 && C > tridiag_cluster_size(esz, n) && C > 8 && C > max_cluster()) return AGB_ERR_UNSUPPORTED;
   g_tuned_C[esz == 16][(n + 31) / 32][count_class(count)] = C;
   g_tuned_T[esz == 16][(n + 31) / 32][count_class(count)] = C > 0 ? threads : 0;
   return AGB_OK;

@@ -143,14 +143,14 @@ __global__ void setup_kernel(int64_t* __restrict__ desc, int ng, char* ws, int e
   gr.lda = n; gr.ldb = n; gr.ldd = n; gr.ldc = n;
   gr.M = n; gr.N = n; gr.K = m;
   gr.opA = 2; gr.opB = 0;
-  gr.alpha_re = 1; gr.alpha_im = 0; gr.beta_re = 0; gr.beta_im = 0;
+  gr.alpha_re = 1; gr.alpha_im = 0; gr.beta_re = 0; gr.beta_im = 0; gr.eye = 0;
   gp[2 * ng + g] = gr;
   GemmProb av;
   av.A = slab + L.X; av.B = slab + L.V; av.D = slab + L.AV; av.Csrc = slab + L.AV;
   av.lda = n; av.ldb = ell; av.ldd = ell; av.ldc = ell;
   av.M = m; av.N = ell; av.K = n;
   av.opA = 0; av.opB = 0;
-  av.alpha_re = 1; av.alpha_im = 0; av.beta_re = 0; av.beta_im = 0;
+  av.alpha_re = 1; av.alpha_im = 0; av.beta_re = 0; av.beta_im = 0; av.eye = 0;
   gp[3 * ng + g] = av;
   ContractProb c;
   c.A = (const void*)D[AGB_D_A];
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(1024) rank_kernel(int64_t* __restrict__ desc, 
     status = AGB_ERR_NOCONV;
     k = 0;
   }
-  if (hp[g].fail) {  // a bounded wait of the band stage expired
+  if (hp[g].fail) {  // a bounded wait of the tridiagonalisation expired
     status = AGB_ERR_TIMEOUT;
     k = 0;
   }
