@@ -22,8 +22,13 @@
 //    the same order as twelve N=64 MMAs would), k slices rotating over four
 //    accumulator pairs; a commit per stage frees the stage for the converters;
 //  * warps 0-7 then read the accumulators with tcgen05.ld (warp w reads TMEM
-//    lanes 32(w%4)..+31 = tile rows, columns 32(w/4)..+31) and write
-//    alpha*C + beta*Csrc.
+//    lanes 32(w%4)..+31 = tile rows, columns 32(w/4)..+31), turn their blocks
+//    in shared memory and write alpha*C + beta*Csrc in whole row pieces.
+// What bounds it: shared-memory bandwidth.  A slice moves 112 KiB of converter
+// stores, 192 KiB of operand reads by its 24 MMAs and 96 KiB of global loads
+// through the SM's 128 B/clk: 3100 cycles, as measured (24 MMAs alone: 1900).
+// 16384 x 512 x 256 (one site of 16 384 shots at chi 256): 118 us a launch, 152
+// before the epilogue's turn, the once-formed addresses and the one-slice read-ahead.
 // The operands are read once per tile and never written back in split form:
 // no packing pass and no packed copy in global memory.  The converters'
 // shared-memory stores reach the tensor core through fence.proxy.async and the
@@ -99,16 +104,13 @@ AGB_DEV void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-AGB_DEV void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
+// 16 columns of the warp's 32 lanes; valid after the next wait::ld.
+AGB_DEV void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // x rounded to TF32 (10 explicit mantissa bits), round to nearest even.
@@ -154,38 +156,73 @@ AGB_DEV void quad_coord(bool k_contig, int ct, int j, int& r, int& k4) {
 //   A (which 0): op(A)[row][k];  B (which 1): op(B)[k][row]
 // stored form: A op N/R -> A[row][k]; op T/C -> A[k][row]
 //              B op N/R -> B[k][row]; op T/C -> B[row][k]
+// A converter thread reads NQ quads of every k slice.  Their addresses are
+// formed once and advance by a constant per slice: with the address
+// arithmetic and the bounds checks of each element inside the loop, a slice cost
+// ~40 instructions per element and the tensor pipe was 31% active.
+template <int NQ>
 struct Operand {
-  const float2* p;
-  int64_t ld;
-  int rows, K;
-  bool k_contig, conj;
+  const float2* q[NQ];  // quad j of the next slice
+  int64_t kstride, step;  // elements between consecutive k, and between slices
+  int K;
+  bool row_ok[NQ], k_contig, vec, conj;
 };
-AGB_DEV Operand operand(const GemmProb& P, int which) {
-  Operand o;
+template <int NQ>
+AGB_DEV Operand<NQ> operand(const GemmProb& P, int which, int r0, int ct) {
+  Operand<NQ> o;
   const int op = which == 0 ? P.opA : P.opB;
-  o.p = (const float2*)(which == 0 ? P.A : P.B);
-  o.ld = which == 0 ? P.lda : P.ldb;
-  o.rows = which == 0 ? P.M : P.N;
-  o.K = P.K;
+  const float2* p = (const float2*)(which == 0 ? P.A : P.B);
+  const int64_t ld = which == 0 ? P.lda : P.ldb;
+  const int rows = which == 0 ? P.M : P.N;
   const bool transposed = (op == 1 || op == 2);
+  o.K = P.K;
   o.k_contig = (which == 0) ? !transposed : transposed;
   o.conj = (op == 2 || op == 3);
-  return o;
-}
-template <int NQ>
-AGB_DEV void load_slice(const Operand& o, int r0, int k0, int ct, float2* v) {
+  o.kstride = o.k_contig ? 1 : ld;
+  o.step = BK * o.kstride;
+  // a quad of consecutive k is two 16-byte loads where every row starts on 16 bytes
+  o.vec = o.k_contig && ((uintptr_t)p & 15) == 0 && (ld & 1) == 0;
 #pragma unroll
   for (int j = 0; j < NQ; ++j) {
     int r, k4;
     quad_coord(o.k_contig, ct, j, r, k4);
-    r += r0;
+    o.row_ok[j] = r0 + r < rows;
+    const int rr = o.row_ok[j] ? r0 + r : 0;
+    o.q[j] = o.k_contig ? p + (int64_t)rr * ld + k4 : p + (int64_t)k4 * ld + rr;
+  }
+  return o;
+}
+template <int NQ>
+AGB_DEV void load_slice(Operand<NQ>& o, int k0, int ct, float2* v) {
+  const float2 zero = make_float2(0.f, 0.f);
+  const bool full = k0 + BK <= o.K;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int k = k0 + k4 + t;
-      float2 x = make_float2(0.f, 0.f);
-      if (r < o.rows && k < o.K) x = o.k_contig ? o.p[(int64_t)r * o.ld + k] : o.p[(int64_t)k * o.ld + r];
-      v[4 * j + t] = x;
+  for (int j = 0; j < NQ; ++j) {
+    float2* d = v + 4 * j;
+    const float2* q = o.q[j];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) d[t] = zero;
+    if (o.row_ok[j]) {
+      if (full) {
+        if (o.vec) {
+          const float4 a = *(const float4*)q, b = *(const float4*)(q + 2);
+          d[0] = make_float2(a.x, a.y);
+          d[1] = make_float2(a.z, a.w);
+          d[2] = make_float2(b.x, b.y);
+          d[3] = make_float2(b.z, b.w);
+        } else {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) d[t] = q[t * o.kstride];
+        }
+      } else {
+        int r, k4;
+        quad_coord(o.k_contig, ct, j, r, k4);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          if (k0 + k4 + t < o.K) d[t] = q[t * o.kstride];
+      }
     }
+    o.q[j] = q + o.step;
   }
 }
 // B quads: the hi and lo planes hold rows [-Im | Re | Im] (BN rows each), so
@@ -193,7 +230,7 @@ AGB_DEV void load_slice(const Operand& o, int r0, int k0, int ct, float2* v) {
 // 0..2BN-1 the operand [-Im | Re] of an A_im product: one N = 2 BN MMA then
 // accumulates both the real and the imaginary part of the tile.
 template <int NQ>
-AGB_DEV void store_slice_b(const Operand& o, uint32_t tile, int ct, const float2* v) {
+AGB_DEV void store_slice_b(const Operand<NQ>& o, uint32_t tile, int ct, const float2* v) {
 #pragma unroll
   for (int j = 0; j < NQ; ++j) {
     int r, k4;
@@ -218,7 +255,7 @@ AGB_DEV void store_slice_b(const Operand& o, uint32_t tile, int ct, const float2
   }
 }
 template <int NQ>
-AGB_DEV void store_slice(const Operand& o, uint32_t tile, int plane_bytes, int ct, const float2* v) {
+AGB_DEV void store_slice(const Operand<NQ>& o, uint32_t tile, int plane_bytes, int ct, const float2* v) {
 #pragma unroll
   for (int j = 0; j < NQ; ++j) {
     int r, k4;
@@ -241,9 +278,26 @@ AGB_DEV void store_slice(const Operand& o, uint32_t tile, int plane_bytes, int c
 }
 
 // ------------------------------------------------------------------ GEMM
+// Problems from device memory, or (probs null) a strided batch passed by value.
+struct StridedProbs {
+  GemmProb base;
+  int64_t sA, sB, sC;  // element strides between batch entries
+};
+AGB_DEV GemmProb get_prob(const GemmProb* probs, const StridedProbs& sp) {
+  if (probs) return probs[blockIdx.z];
+  GemmProb p = sp.base;
+  const int64_t z = blockIdx.z;
+  p.A = (const float2*)p.A + z * sp.sA;
+  p.B = (const float2*)p.B + z * sp.sB;
+  p.D = (float2*)p.D + z * sp.sC;
+  p.Csrc = (const float2*)p.Csrc + z * sp.sC;
+  return p;
+}
+
 __global__ void __launch_bounds__(NTHREADS, 1)
-    tc_gemm_kernel(const GemmProb* __restrict__ probs, int* __restrict__ status, unsigned pipe_limit) {
-  const GemmProb P = probs[blockIdx.z];
+    tc_gemm_kernel(const GemmProb* __restrict__ probs, const __grid_constant__ StridedProbs sp,
+                   int* __restrict__ status, unsigned pipe_limit) {
+  const GemmProb P = get_prob(probs, sp);
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   if (m0 >= P.M || n0 >= P.N) return;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -255,9 +309,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = (P.K + BK - 1) / BK;
+  // the first slice's loads are in flight while the barriers and TMEM are set up
+  const int ct = threadIdx.x;
+  Operand<QA> oa;
+  Operand<QB> ob;
+  float2 va[2][4 * QA], vb[2][4 * QB];
+  if (warp < CONV_WARPS) {
+    oa = operand<QA>(P, 0, m0, ct);
+    ob = operand<QB>(P, 1, n0, ct);
+    if (nk > 0) {
+      load_slice<QA>(oa, 0, ct, va[0]);
+      load_slice<QB>(ob, 0, ct, vb[0]);
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], NCONV);
+      mbar_init(&full[s], CONV_WARPS);
       mbar_init(&empty[s], 1);
     }
     mbar_init(done, 1);
@@ -275,23 +342,32 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const uint32_t tmem = *tmem_slot;
   if (warp < CONV_WARPS) {
     // ---------------- converters: global complex64 -> split TF32 planes in shared memory
-    const int ct = threadIdx.x;
-    const Operand oa = operand(P, 0), ob = operand(P, 1);
-    for (int kt = 0; kt < nk; ++kt) {
-      const int s = kt % STAGES;
-      float2 va[4 * QA], vb[4 * QB];
-      load_slice<QA>(oa, m0, kt * BK, ct, va);  // in flight while the stage drains
-      load_slice<QB>(ob, n0, kt * BK, ct, vb);
-      if (kt >= STAGES && !mbar_wait(&empty[s], ((kt / STAGES) - 1) & 1, pipe_limit)) {
-        *abort_flag = 1;
-        break;
+    // slice kt + 1 is read from global memory while slice kt is converted
+    bool stopped = false;
+    for (int kt0 = 0; kt0 < nk && !stopped; kt0 += 2) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int kt = kt0 + u, s = u;  // STAGES == 2: slice kt uses stage kt % 2
+        if (kt >= nk || stopped) break;
+        if (kt + 1 < nk) {
+          load_slice<QA>(oa, (kt + 1) * BK, ct, va[u ^ 1]);
+          load_slice<QB>(ob, (kt + 1) * BK, ct, vb[u ^ 1]);
+        }
+        // one decision per warp: its lanes meet again at the __syncwarp below
+        bool go = kt < STAGES || mbar_wait(&empty[s], ((kt / STAGES) - 1) & 1, pipe_limit);
+        if (!go) *abort_flag = 1;
+        go = go && !*abort_flag;
+        if (!__all_sync(0xffffffffu, go)) {
+          stopped = true;
+          break;
+        }
+        const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
+        store_slice<QA>(oa, st, TILE_A, ct, va[u]);
+        store_slice_b<QB>(ob, st + 4 * TILE_A, ct, vb[u]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor core
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[s]);
       }
-      if (*abort_flag) break;
-      const uint32_t st = smem_u32(smem + s * STAGE_BYTES);
-      store_slice<QA>(oa, st, TILE_A, ct, va);
-      store_slice_b<QB>(ob, st + 4 * TILE_A, ct, vb);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor core
-      mbar_arrive(&full[s]);
     }
   } else if (lane == 0) {
     // ---------------- MMA issuer
@@ -343,8 +419,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const bool ok = mbar_wait(done, 0);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp < CONV_WARPS && ok && !*abort_flag) {
-    const int quarter = warp & 3, half = warp >> 2;  // TMEM lanes 32 quarter.., columns 32 half..
-    const int row = m0 + quarter * 32 + lane;
+    // Warp (quarter, half) reads TMEM lanes 32 quarter.. and columns 32 half..,
+    // one tile row per lane, and turns its 32 x 32 block in shared memory (the
+    // stages are free), so that the global accesses are whole 256-byte row pieces.
+    // Stored straight from the TMEM layout, a store touched 32 rows with 8 bytes
+    // each: 13 800 of a 16 384 x 512 x 256 tile's 44 800 cycles, and the loads of
+    // the other CTAs waited behind it.
+    const int quarter = warp & 3, half = warp >> 2;
+    const int row0 = m0 + quarter * 32, col = n0 + half * (BN / 2) + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     float2* D = (float2*)P.D;
     const float2* C = (const float2*)P.Csrc;
@@ -352,40 +434,57 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const float eye = (float)P.eye;
     const bool use_beta = (br != 0.f || bi != 0.f);
     const int nacc = nk < NACC ? nk : NACC;
+    constexpr int PITCH = BN / 2 + 1;
+    float2* buf = (float2*)smem + warp * 32 * PITCH;
 #pragma unroll 1
-    for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
-      float re[16], im[16];
-      tmem_ld16(tmem + lane_base + c0, re);
-      tmem_ld16(tmem + lane_base + BN + c0, im);
-      if (nk == 0) {
+    for (int c0 = 0; c0 < BN / 2; c0 += 16) {
+      const uint32_t tc = tmem + lane_base + (uint32_t)(half * (BN / 2) + c0);
+      float re[NACC][16], im[NACC][16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) re[i] = im[i] = 0.f;  // empty inner dimension: product is zero
-      }
-      for (int a = 1; a < nacc; ++a) {
-        float r2[16], i2[16];
-        tmem_ld16(tmem + lane_base + (uint32_t)(2 * BN * a) + c0, r2);
-        tmem_ld16(tmem + lane_base + (uint32_t)(2 * BN * a) + BN + c0, i2);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          re[i] += r2[i];
-          im[i] += i2[i];
+      for (int a = 0; a < NACC; ++a)
+        if (a < nacc) {
+          tmem_ld16(tc + (uint32_t)(2 * BN * a), re[a]);
+          tmem_ld16(tc + (uint32_t)(2 * BN * a) + BN, im[a]);
         }
-      }
-      if (row < P.M) {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      // the values count as written here: no use of them moves ahead of the wait
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int col = n0 + c0 + i;
-          if (col < P.N) {
-            float2 v = make_float2(ar * re[i] - ai * im[i], ar * im[i] + ai * re[i]);
-            if (use_beta) {
-              const float2 c = C[(int64_t)row * P.ldc + col];
-              v.x += br * c.x - bi * c.y;
-              v.y += br * c.y + bi * c.x;
-            }
-            if (row == col) v.x += eye;
-            D[(int64_t)row * P.ldd + col] = v;
+      for (int a = 0; a < NACC; ++a)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(re[a][i]), "+f"(im[a][i]));
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float x = 0.f, y = 0.f;  // empty inner dimension: product is zero
+#pragma unroll
+        for (int a = 0; a < NACC; ++a)
+          if (a < nacc) {
+            x = a ? x + re[a][i] : re[a][i];
+            y = a ? y + im[a][i] : im[a][i];
           }
+        buf[lane * PITCH + c0 + i] = make_float2(ar * x - ai * y, ar * y + ai * x);
+      }
+    }
+    __syncwarp();
+    const int nrow = min(32, P.M - row0);
+    if (col < P.N) {
+      float2* d = D + (int64_t)row0 * P.ldd + col;
+      const float2* c = C + (int64_t)row0 * P.ldc + col;
+      const float2* b = buf + lane;
+      if (use_beta || eye != 0.f) {
+#pragma unroll 4
+        for (int r = 0; r < nrow; ++r, d += P.ldd, c += P.ldc, b += PITCH) {
+          float2 v = *b;
+          if (use_beta) {
+            const float2 z = *c;
+            v.x += br * z.x - bi * z.y;
+            v.y += br * z.y + bi * z.x;
+          }
+          if (row0 + r == col) v.x += eye;
+          *d = v;
         }
+      } else {
+#pragma unroll 8
+        for (int r = 0; r < nrow; ++r, d += P.ldd, b += PITCH) *d = *b;
       }
     }
   } else if (threadIdx.x == 0 && (!ok || *abort_flag)) {
@@ -422,8 +521,8 @@ size_t tc_gemm_scratch_bytes(int count, int maxM, int maxN, int maxK) {
   return 256;
 }
 
-int launch_gemm_tc(const GemmProb* probs, int count, int maxM, int maxN, int maxK, void* scratch,
-                   size_t scratch_bytes, int* status, cudaStream_t s) {
+static int launch_tc(const GemmProb* probs, const StridedProbs& sp, int count, int maxM, int maxN, int maxK,
+                     void* scratch, size_t scratch_bytes, int* status, cudaStream_t s) {
   if (count <= 0 || maxM <= 0 || maxN <= 0) return AGB_OK;
   if (maxK <= 0) return AGB_ERR_ARG;
   if (count > 65535) return AGB_ERR_UNSUPPORTED;
@@ -435,23 +534,20 @@ int launch_gemm_tc(const GemmProb* probs, int count, int maxM, int maxN, int max
       return AGB_ERR_CUDA;
     attr = true;
   }
-  tc_gemm_kernel<<<dim3(Np / BN, Mp / BM, count), NTHREADS, SMEM_BYTES, s>>>(probs, status, g_pipe_limit);
+  tc_gemm_kernel<<<dim3(Np / BN, Mp / BM, count), NTHREADS, SMEM_BYTES, s>>>(probs, sp, status, g_pipe_limit);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }
 
+int launch_gemm_tc(const GemmProb* probs, int count, int maxM, int maxN, int maxK, void* scratch,
+                   size_t scratch_bytes, int* status, cudaStream_t s) {
+  if (!probs) return AGB_ERR_ARG;
+  const StridedProbs none = {};
+  return launch_tc(probs, none, count, maxM, maxN, maxK, scratch, scratch_bytes, status, s);
+}
+
 // Strided-batch host entry for the tensor-core GEMM (complex64).
 namespace {
-__global__ void strided_probs_kernel(GemmProb* out, GemmProb base, int count, int64_t sA, int64_t sB, int64_t sC) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  GemmProb p = base;
-  p.A = (const float2*)base.A + (int64_t)i * sA;
-  p.B = (const float2*)base.B + (int64_t)i * sB;
-  p.D = (float2*)base.D + (int64_t)i * sC;
-  p.Csrc = (const float2*)base.Csrc + (int64_t)i * sC;
-  out[i] = p;
-}
 int opc(char c) {
   return (c == 'N' || c == 'n') ? 0 : (c == 'T' || c == 't') ? 1 : (c == 'C' || c == 'c') ? 2 : (c == 'R' || c == 'r') ? 3 : -1;
 }
@@ -473,7 +569,8 @@ static int cgemm_tc_impl(char opA, char opB, int batch, int M, int N, int K, con
   if (oa < 0 || ob < 0 || batch < 0 || M < 0 || N < 0 || K <= 0 || !ws) return AGB_ERR_ARG;
   if (batch == 0 || M == 0 || N == 0) return AGB_OK;
   if (ws_bytes < agb_cgemm_tc_workspace(batch, M, N, K)) return AGB_ERR_WORKSPACE;
-  GemmProb base;
+  StridedProbs sp;
+  GemmProb& base = sp.base;
   base.A = A;
   base.B = B;
   base.D = C;
@@ -493,15 +590,15 @@ static int cgemm_tc_impl(char opA, char opB, int batch, int M, int N, int K, con
   base.beta_im = beta_im;
   base.eye = 0;
   char* w = (char*)ws;
-  GemmProb* probs = (GemmProb*)w;
+  sp.sA = strideA;
+  sp.sB = strideB;
+  sp.sC = strideC;
   int* status = (int*)(w + agb_align((size_t)batch * sizeof(GemmProb)));
   void* scratch = w + agb_align((size_t)batch * sizeof(GemmProb)) + agb_align(sizeof(int));
   cudaStream_t s = (cudaStream_t)stream;
   if (status_dev) status = status_dev;
   else if (cudaMemsetAsync(status, 0, sizeof(int), s) != cudaSuccess) return AGB_ERR_CUDA;
-  strided_probs_kernel<<<(batch + 127) / 128, 128, 0, s>>>(probs, base, batch, strideA, strideB, strideC);
-  AGB_CHECK_LAUNCH();
-  int rc = launch_gemm_tc(probs, batch, M, N, K, scratch, ws_bytes - (size_t)((char*)scratch - w), status, s);
+  int rc = launch_tc(nullptr, sp, batch, M, N, K, scratch, ws_bytes - (size_t)((char*)scratch - w), status, s);
   if (rc) return rc;
   if (status_host && !status_dev) {
     if (cudaMemcpyAsync(status_host, status, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return AGB_ERR_CUDA;
