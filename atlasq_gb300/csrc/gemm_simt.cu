@@ -1,12 +1,18 @@
-// SIMT batched complex GEMM for sm_103a: 64x64 output tiles, K-step 8,
-// 256 threads, 4x4 complex accumulators per thread.  Used for small and ragged
-// shapes, and for complex128.
+// SIMT batched complex GEMM for sm_103a, 256 threads.  complex64: 64 x 64 output
+// tiles, K-step 8, 4 x 4 complex accumulators per thread (small and ragged
+// shapes).  complex128: 16 x 16 tiles, K-step 16, one output per thread: the
+// FP64 pipe does 2 lanes per clock and SM whatever the tile, so what counts is
+// how many SMs a product spreads over and how little of a ragged tile is
+// padding (a 10-gate layer at chi 48: 189 us over its 19 launches, 2043 us with
+// 64 x 64 tiles, 40 CTAs a launch and a third of their area padding).
 #include "gemm.cuh"
 #include "gemm_tc.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 8;
+template <typename CX> struct Tile;
+template <> struct Tile<float2> { static constexpr int B = 64, K = 8, T = 4; };
+template <> struct Tile<double2> { static constexpr int B = 16, K = 16, T = 1; };
 
 template <typename CX>
 AGB_DEV CX load_op(const CX* P, int64_t ld, int op, int row, int col, int rows, int cols) {
@@ -36,9 +42,11 @@ AGB_DEV GemmProb get_prob(const GemmProb* probs, const StridedBatch& sb) {
 }
 
 template <typename CX>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restrict__ probs, StridedBatch sb) {
+__global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restrict__ probs, StridedBatch sb,
+                                                        int tiles_n) {
+  constexpr int BM = Tile<CX>::B, BN = Tile<CX>::B, BK = Tile<CX>::K, T = Tile<CX>::T;
   const GemmProb p = get_prob<CX>(probs, sb);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int m0 = (int)(blockIdx.x / tiles_n) * BM, n0 = (int)(blockIdx.x % tiles_n) * BN;
   if (m0 >= p.M || n0 >= p.N) return;
   typedef typename cx_traits<CX>::R R;
   __shared__ CX As[BK][BM + 1];
@@ -46,16 +54,16 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const CX* A = (const CX*)p.A;
   const CX* B = (const CX*)p.B;
-  CX acc[4][4];
+  CX acc[T][T];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < T; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = czero<CX>();
+    for (int j = 0; j < T; ++j) acc[i][j] = czero<CX>();
 
   for (int k0 = 0; k0 < p.K; k0 += BK) {
     // A tile: BM x BK of op(A); B tile: BK x BN of op(B)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
+    for (int e = 0; e < BM * BK / 256; ++e) {
       const int idx = tid + e * 256;
       int r, c;
       if (p.opA == 0 || p.opA == 3) { r = idx / BK; c = idx % BK; } else { r = idx % BM; c = idx / BM; }
@@ -65,17 +73,22 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
       Bs[kr][nc] = load_op(B, p.ldb, p.opB, k0 + kr, n0 + nc, p.K, p.N);
     }
     __syncthreads();
+    const int kn = min(BK, p.K - k0);
+    if (T == 1 && kn < BK) {  // no padding products on the FP64 pipe
+      for (int k = 0; k < kn; ++k) cfma(acc[0][0], As[k][ty], Bs[k][tx]);
+    } else {
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      CX a[4], b[4];
+      for (int k = 0; k < BK; ++k) {
+        CX a[T], b[T];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty + 16 * i];
+        for (int i = 0; i < T; ++i) a[i] = As[k][ty + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[k][tx + 16 * j];
+        for (int j = 0; j < T; ++j) b[j] = Bs[k][tx + 16 * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < T; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) cfma(acc[i][j], a[i], b[j]);
+          for (int j = 0; j < T; ++j) cfma(acc[i][j], a[i], b[j]);
+      }
     }
     __syncthreads();
   }
@@ -85,11 +98,11 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
   CX* D = (CX*)p.D;
   const CX* C = (const CX*)p.Csrc;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < T; ++i) {
     const int r = m0 + ty + 16 * i;
     if (r >= p.M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < T; ++j) {
       const int c = n0 + tx + 16 * j;
       if (c >= p.N) continue;
       CX v = cmul(alpha, acc[i][j]);
@@ -109,9 +122,11 @@ int launch_gemm_probs(const GemmProb* probs, int count, int maxM, int maxN, cuda
   if (sizeof(CX) == 8 && ctx && ctx->tc_scratch && maxM >= 64 && maxN >= 64 && maxK >= 32 &&
       ctx->tc_bytes >= tc_gemm_scratch_bytes(count, maxM, maxN, maxK))
     return launch_gemm_tc(probs, count, maxM, maxN, maxK, ctx->tc_scratch, ctx->tc_bytes, ctx->status, s);
-  dim3 grid((maxN + BN - 1) / BN, (maxM + BM - 1) / BM, count);
+  constexpr int B = Tile<CX>::B;
+  const int tn = (maxN + B - 1) / B, tm = (maxM + B - 1) / B;
+  if ((int64_t)tn * tm > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
   StridedBatch sb = {};
-  gemm_simt_kernel<CX><<<grid, 256, 0, s>>>(probs, sb);
+  gemm_simt_kernel<CX><<<dim3(tn * tm, 1, count), 256, 0, s>>>(probs, sb, tn);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }
@@ -162,11 +177,14 @@ extern "C" int agb_cgemm_batched(int dtype, char opA, char opB, int batch, int M
   sb.sB = strideB;
   sb.sC = strideC;
   cudaStream_t s = (cudaStream_t)stream;
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
+  const int B_ = dtype == AGB_C64 ? Tile<float2>::B : Tile<double2>::B;
+  const int64_t tn = ((int64_t)N + B_ - 1) / B_, tm = ((int64_t)M + B_ - 1) / B_;
+  if (tn * tm > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)(tn * tm), 1, batch);
   if (dtype == AGB_C64)
-    gemm_simt_kernel<float2><<<grid, 256, 0, s>>>(nullptr, sb);
+    gemm_simt_kernel<float2><<<grid, 256, 0, s>>>(nullptr, sb, (int)tn);
   else
-    gemm_simt_kernel<double2><<<grid, 256, 0, s>>>(nullptr, sb);
+    gemm_simt_kernel<double2><<<grid, 256, 0, s>>>(nullptr, sb, (int)tn);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }

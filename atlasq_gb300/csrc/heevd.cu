@@ -233,11 +233,14 @@ AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
   return cnt;
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) bisect_kernel(const HeevdProb* __restrict__ probs) {
+// A warp per eigenvalue, WARPS of them per CTA: 8 for float; 2 for double, whose
+// divisions are bound by the FP64 pipe of the SM (10 problems of n = 96: 499 us,
+// 918 us on the 60 CTAs of 8 warps).
+template <typename R, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __restrict__ probs) {
   const HeevdProb P = probs[blockIdx.y];
   const int n = P.n, ell = P.ell;
-  if (blockIdx.x * 8 >= ell) return;
+  if (blockIdx.x * WARPS >= ell) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* d = (R*)smem_raw;
   R* e2 = d + n;
@@ -249,12 +252,18 @@ __global__ void __launch_bounds__(256) bisect_kernel(const HeevdProb* __restrict
     e2[i] = (i < n - 1) ? eg[i] * eg[i] : R(0);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // Gershgorin interval (min and max do not depend on the order)
+  if (threadIdx.x < 32) {
     R gl = d[0], gu = d[0];
-    for (int i = 0; i < n; ++i) {
+    for (int i = threadIdx.x; i < n; i += 32) {
       const R r = (i > 0 ? fabs(eg[i - 1]) : R(0)) + (i < n - 1 ? fabs(eg[i]) : R(0));
       gl = fmin(gl, d[i] - r);
       gu = fmax(gu, d[i] + r);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
+      gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
     }
     const R span = fmax(fabs(gl), fabs(gu));
     glim[0] = gl - R(4) * rlim<R>::eps() * span - rlim<R>::pivmin();
@@ -262,7 +271,7 @@ __global__ void __launch_bounds__(256) bisect_kernel(const HeevdProb* __restrict
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int t = blockIdx.x * 8 + wid;
+  const int t = blockIdx.x * WARPS + wid;
   if (t >= ell) return;
   const int idx = n - 1 - t;  // ascending index of the t-th largest eigenvalue
   R lo = glim[0], hi = glim[1];
@@ -1272,7 +1281,8 @@ int launch_heevd_values(HeevdProb* probs, int count, int maxn, int maxell, cudaS
   if (maxell <= 0) return AGB_OK;
   const size_t sm_r = 2 * (size_t)maxn * sizeof(R);
   prof_mark(AGB_ST_BISECT, s);
-  bisect_kernel<R><<<dim3((maxell + 7) / 8, count), 256, sm_r, s>>>(probs);
+  constexpr int BW = sizeof(R) == 8 ? 2 : 8;
+  bisect_kernel<R, BW><<<dim3((maxell + BW - 1) / BW, count), 32 * BW, sm_r, s>>>(probs);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }

@@ -326,22 +326,25 @@ static bool cluster_fits(int esz, int n, int C) {
 
 // Pick the cluster size for a matrix of size n: the autotuned choice for this
 // size and batch class if there is one; otherwise for complex64 the register
-// form's own rule, for complex128 the smallest of 1..8 CTAs whose shared memory
-// holds every row (at least 8 above n = 256, where the per-step work, not the
-// barriers, dominates); else the largest cluster the device schedules, with
-// the overflow rows in L2.
+// form's own rule.  complex128 is bound by the FP64 pipe (2 lanes per clock and
+// SM), so a matrix takes 8 CTAs as soon as it has a few rows for each (10
+// matrices of n = 96: 1.25 ms on 8 CTAs, 1.45 on 4, 2.91 on 1; 4 of n = 160: 2.6
+// against 8.2; 10 of n = 24: 0.25 on 4 or 8, 0.32 on 1), fewer when the batch
+// fills the SMs by itself and every row still fits; where the rows do not fit
+// 8 CTAs, the largest cluster the device schedules, with the overflow rows in L2.
 int tridiag_cluster_size_for(int esz, int n, int count) {
   const int t = g_tuned_C[esz == 16][(n + 31) / 32][count_class(count)];
   if (t > 0 && cluster_fits(esz, n, t)) return t;
   if (esz == 8) return tridiag_reg_ctas(n, count);
-  return tridiag_cluster_size(esz, n);
+  int C = tridiag_cluster_size(esz, n);
+  while (C > 1 && C <= 8 && C * count > 152 && tridiag_cluster_smem(esz, n, C / 2) <= kSmemBudget) C /= 2;
+  return C;
 }
 
 int tridiag_cluster_size(int esz, int n) {
   if (esz == 8) return tridiag_reg_ctas(n, 1);
-  const int lo = n > 256 ? 8 : 1;
-  for (int C = lo; C <= 8; ++C)
-    if (tridiag_cluster_smem(esz, n, C) <= kSmemBudget) return C;
+  const int C = n <= 8 ? 1 : n <= 32 ? 4 : 8;
+  if (tridiag_cluster_smem(esz, n, C) <= kSmemBudget) return C;
   if (6 * (size_t)n * esz + 64 * 1024 > kSmemBudget) return 0;
   return max_cluster();
 }

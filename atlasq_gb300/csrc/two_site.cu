@@ -165,67 +165,122 @@ __global__ void setup_kernel(int64_t* __restrict__ desc, int ng, char* ws, int e
 }
 
 // ------------------------------------------------------------------ contraction
-// Tile: 16 left indices l x 16 right indices j, all four (p', q'), K-chunks of 16.
-template <typename CX>
-__global__ void __launch_bounds__(256) contract_gate_kernel(const ContractProb* __restrict__ probs,
-                                                            ContractProb single) {
+// Tile: TL left indices l x TL right indices j, all four (p', q'), K-chunks of
+// 16.  A thread takes S x S of the tile's (l, j) (16 outputs for S = 2), so a
+// K step reads 2 S pairs from shared memory for 16 S S multiply-adds.  complex128
+// takes 8 x 8 tiles of 64 threads: bound by the FP64 pipe, it wants many SMs.
+// The sum over r runs in the same order whatever the tile.  Bound by the
+// latency of a chunk (load, barrier, 16 steps), hence the read-ahead: chi 256
+// alone 20.5 us (25.9 before), chi 100 6.8 (10.7), a 20-gate chi 256 layer 90 (110).
+template <typename CX, int TL, int S>
+__global__ void __launch_bounds__((TL / S) * (TL / S)) contract_gate_kernel(const ContractProb* __restrict__ probs,
+                                                                            ContractProb single) {
+  constexpr int W = TL / S, NT = W * W, KC = 16;
+  struct __align__(2 * sizeof(CX)) Pair { CX a, b; };
   const ContractProb P = probs ? probs[blockIdx.z] : single;
-  const int l0 = blockIdx.y * 16, j0 = blockIdx.x * 16;
+  const int l0 = blockIdx.y * TL, j0 = blockIdx.x * TL;
   if (l0 >= P.chiL || j0 >= P.chiR) return;
-  __shared__ CX As[16][2][17];
-  __shared__ CX Bs[16][2][17];
+  __shared__ Pair As[KC][TL + 1];  // [r][l]: p' = 0, 1 side by side
+  __shared__ Pair Bs[KC][TL + 1];  // [r][j]: q' = 0, 1
   __shared__ CX Us[16];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, tx = tid % W, ty = tid / W;
   const CX* A = (const CX*)P.A;
   const CX* B = (const CX*)P.B;
   if (tid < 16) Us[tid] = ((const CX*)P.U)[tid];
-  CX th[2][2];
-  th[0][0] = th[0][1] = th[1][0] = th[1][1] = czero<CX>();
-  const int chiM = P.chiM, chiR = P.chiR, chiL = P.chiL;
-  for (int r0 = 0; r0 < chiM; r0 += 16) {
+  CX th[S][S][2][2];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int idx = tid + 256 * e;  // 0..511
-      // A[l][p][r]: l = idx / 32, p = (idx / 16) % 2, r = idx % 16
-      {
-        const int l = idx >> 5, pp = (idx >> 4) & 1, r = idx & 15;
+  for (int a = 0; a < S; ++a)
+#pragma unroll
+    for (int b = 0; b < S; ++b) th[a][b][0][0] = th[a][b][0][1] = th[a][b][1][0] = th[a][b][1][1] = czero<CX>();
+  const int chiM = P.chiM, chiR = P.chiR, chiL = P.chiL;
+  // the next chunk is read into registers while the current one is multiplied
+  constexpr int NE = 2 * TL * KC / NT;
+  CX va[NE], vb[NE];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int idx = tid + NT * e;
+      {  // A[l][p][r]: r fastest
+        const int r = idx % KC, pp = (idx / KC) & 1, l = idx / (2 * KC);
         const int gl = l0 + l, gr = r0 + r;
-        As[l][pp][r] = (gl < chiL && gr < chiM) ? A[((int64_t)gl * 2 + pp) * chiM + gr] : czero<CX>();
+        va[e] = (gl < chiL && gr < chiM) ? A[((int64_t)gl * 2 + pp) * chiM + gr] : czero<CX>();
       }
-      // B[r][q][j]: r = idx / 32, q = (idx / 16) % 2, j = idx % 16
-      {
-        const int r = idx >> 5, q = (idx >> 4) & 1, j = idx & 15;
+      {  // B[r][q][j]: j fastest
+        const int j = idx % TL, qq = (idx / TL) & 1, r = idx / (2 * TL);
         const int gr = r0 + r, gj = j0 + j;
-        Bs[r][q][j] = (gr < chiM && gj < chiR) ? B[((int64_t)gr * 2 + q) * chiR + gj] : czero<CX>();
+        vb[e] = (gr < chiM && gj < chiR) ? B[((int64_t)gr * 2 + qq) * chiR + gj] : czero<CX>();
       }
     }
-    __syncthreads();
+  };
+  fetch(0);
+  for (int r0 = 0; r0 < chiM; r0 += KC) {
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      const CX a0 = As[ty][0][r], a1 = As[ty][1][r];
-      const CX b0 = Bs[r][0][tx], b1 = Bs[r][1][tx];
-      cfma(th[0][0], a0, b0);
-      cfma(th[0][1], a0, b1);
-      cfma(th[1][0], a1, b0);
-      cfma(th[1][1], a1, b1);
+    for (int e = 0; e < NE; ++e) {
+      const int idx = tid + NT * e;
+      CX* as = &As[idx % KC][idx / (2 * KC)].a;
+      as[(idx / KC) & 1] = va[e];
+      CX* bs = &Bs[idx / (2 * TL)][idx % TL].a;
+      bs[(idx / TL) & 1] = vb[e];
+    }
+    __syncthreads();
+    if (r0 + KC < chiM) fetch(r0 + KC);
+    const int rn = sizeof(CX) == 16 ? min(KC, chiM - r0) : KC;  // no padding products on the FP64 pipe
+#pragma unroll (sizeof(CX) == 16 ? 1 : KC)
+    for (int r = 0; r < rn; ++r) {
+      Pair a[S], b[S];
+#pragma unroll
+      for (int k = 0; k < S; ++k) {
+        a[k] = As[r][ty + W * k];
+        b[k] = Bs[r][tx + W * k];
+      }
+#pragma unroll
+      for (int i = 0; i < S; ++i)
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+          cfma(th[i][j][0][0], a[i].a, b[j].a);
+          cfma(th[i][j][0][1], a[i].a, b[j].b);
+          cfma(th[i][j][1][0], a[i].b, b[j].a);
+          cfma(th[i][j][1][1], a[i].b, b[j].b);
+        }
     }
     __syncthreads();
   }
-  const int l = l0 + ty, j = j0 + tx;
-  if (l >= chiL || j >= chiR) return;
   CX* X = (CX*)P.X;
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+  for (int i = 0; i < S; ++i)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int row = 2 * p + q;
-      CX acc = czero<CX>();
-      cfma(acc, Us[row * 4 + 0], th[0][0]);
-      cfma(acc, Us[row * 4 + 1], th[0][1]);
-      cfma(acc, Us[row * 4 + 2], th[1][0]);
-      cfma(acc, Us[row * 4 + 3], th[1][1]);
-      X[((int64_t)l * 2 + p) * P.ldx + (int64_t)q * chiR + j] = acc;
+    for (int jj = 0; jj < S; ++jj) {
+      const int l = l0 + ty + W * i, j = j0 + tx + W * jj;
+      if (l >= chiL || j >= chiR) continue;
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int row = 2 * p + q;
+          CX acc = czero<CX>();
+          cfma(acc, Us[row * 4 + 0], th[i][jj][0][0]);
+          cfma(acc, Us[row * 4 + 1], th[i][jj][0][1]);
+          cfma(acc, Us[row * 4 + 2], th[i][jj][1][0]);
+          cfma(acc, Us[row * 4 + 3], th[i][jj][1][1]);
+          X[((int64_t)l * 2 + p) * P.ldx + (int64_t)q * chiR + j] = acc;
+        }
     }
+}
+
+// complex64: 32 x 32 tiles (twice the arithmetic per shared-memory read of 16 x
+// 16: 90 against 111 us for the layer above) where they still make two CTAs per
+// SM; else 16 x 16 (one chi 256 gate has 64 tiles of 32 and 256 of 16).
+template <typename CX>
+void launch_contract(const ContractProb* probs, const ContractProb& single, int maxL, int maxR, int count,
+                     cudaStream_t s) {
+  auto grid = [&](int t) { return dim3((maxR + t - 1) / t, (maxL + t - 1) / t, count); };
+  if constexpr (sizeof(CX) == 16) {
+    contract_gate_kernel<CX, 8, 1><<<grid(8), 64, 0, s>>>(probs, single);
+  } else {
+    const dim3 g = grid(32);
+    if ((int64_t)g.x * g.y * g.z >= 2 * 152) contract_gate_kernel<CX, 32, 2><<<g, 256, 0, s>>>(probs, single);
+    else contract_gate_kernel<CX, 16, 1><<<grid(16), 256, 0, s>>>(probs, single);
+  }
 }
 
 // The reference rank rule (truncation.py:21-83) for one gate, on sigma^2 values
@@ -679,7 +734,7 @@ int run_impl(int ng, int64_t* desc, int maxL, int maxM, int maxR, int maxell, ch
                                      agb_align((size_t)ng * 4 * sizeof(GemmProb)));
   ContractProb none = {};
   prof_mark(AGB_ST_CONTRACT, s);
-  contract_gate_kernel<CX><<<dim3((maxR + 15) / 16, (maxL + 15) / 16, ng), 256, 0, s>>>(cp, none);
+  launch_contract<CX>(cp, none, maxL, maxR, ng, s);
   AGB_CHECK_LAUNCH();
   const int maxm = 2 * maxL, maxn = 2 * maxR;
   GemmCtx ctx;
@@ -740,9 +795,8 @@ extern "C" int agb_contract_gate(int dtype, const void* A, const void* B, const 
   p.chiR = chiR;
   p.ldx = 2 * (int64_t)chiR;
   cudaStream_t s = (cudaStream_t)stream;
-  dim3 grid((chiR + 15) / 16, (chiL + 15) / 16, 1);
-  if (dtype == AGB_C64) contract_gate_kernel<float2><<<grid, 256, 0, s>>>(nullptr, p);
-  else contract_gate_kernel<double2><<<grid, 256, 0, s>>>(nullptr, p);
+  if (dtype == AGB_C64) launch_contract<float2>(nullptr, p, chiL, chiR, 1, s);
+  else launch_contract<double2>(nullptr, p, chiL, chiR, 1, s);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }
