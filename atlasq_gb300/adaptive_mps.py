@@ -30,6 +30,7 @@ from .diagnostics import MPSStatistics
 from .truncation import check_entropy_sanity
 
 _C64, _C128 = torch.complex64, torch.complex128
+_ORTH_GUARD2 = float(np.float32(0.3) * np.float32(0.3))  # kOrthGuard squared (csrc/heevd.cuh)
 
 
 @dataclass
@@ -715,10 +716,19 @@ def _run_pipeline(entries, dt, ells, all_vectors=False, cluster_tol=None, spectr
     stream = stream_ptr(device)
     # a gate whose eigenvalue-guided eigenvector count fell short is re-run with
     # every vector on the device; AGB_ERR_RANK then only means a predicted ell
-    # below the rank, which the caller re-runs at full size
-    check(lib.agb_two_site_run(code, G, ptr(desc_dev), ptr(desc_dev), maxL, maxM, maxR, maxell,
-                               ptr(ws), wsz.value, stream,
-                               _lib.AGB_RUN_REPAIR | (0 if guard else _lib.AGB_RUN_NO_GUARD)), "two_site_run")
+    # below the rank, which the caller re-runs at full size.  The results come
+    # back anyway, so the re-run is issued only when some gate needs it.
+    gflag = 0 if guard else _lib.AGB_RUN_NO_GUARD
+
+    def run(flags):
+        check(lib.agb_two_site_run(code, G, ptr(desc_dev), ptr(desc_dev), maxL, maxM, maxR, maxell,
+                                   ptr(ws), wsz.value, stream, flags | gflag), "two_site_run")
+        return desc_dev.cpu().numpy()
+
+    out = run(_lib.AGB_RUN_REPAIR_LATER)
+    overlap = ~(np.ascontiguousarray(out[:, _lib.D_ORTH]).view(np.float64) <= _ORTH_GUARD2)
+    if (out[:, _lib.D_STATUS] == _lib.AGB_ERR_RANK).any() or (guard and (overlap & (out[:, _lib.D_MODE] == 0)).any()):
+        out = run(_lib.AGB_RUN_REPAIR_ONLY)
     sig = None
     if spectra:
         cnt = max(1, maxell)
@@ -726,7 +736,6 @@ def _run_pipeline(entries, dt, ells, all_vectors=False, cluster_tol=None, spectr
         check(lib.agb_two_site_spectra(code, G, ptr(desc_dev), ptr(ws), cnt, ptr(sig_dev), stream),
               "two_site_spectra")
         sig = sig_dev.cpu().numpy()
-    out = desc_dev.cpu().numpy()
     res = []
     maxk = 1
     sts = out[:, _lib.D_STATUS].tolist()

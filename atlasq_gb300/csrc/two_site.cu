@@ -724,45 +724,50 @@ template <typename CX>
 int run_impl(int ng, int64_t* desc, int maxL, int maxM, int maxR, int maxell, char* ws, size_t ws_bytes,
              size_t tc_bytes, cudaStream_t s, int flags) {
   const int esz = sizeof(CX);
-  if (cudaMemsetAsync(status_word(ws, ng), 0, sizeof(int), s) != cudaSuccess) return AGB_ERR_CUDA;
-  prof_mark(AGB_ST_SETUP, s);
-  setup_kernel<<<(ng + 127) / 128, 128, 0, s>>>(desc, ng, ws, esz);
-  AGB_CHECK_LAUNCH();
   HeevdProb* hp = (HeevdProb*)ws;
   GemmProb* gp = (GemmProb*)(ws + agb_align((size_t)ng * sizeof(HeevdProb)));
-  ContractProb* cp = (ContractProb*)(ws + agb_align((size_t)ng * sizeof(HeevdProb)) +
-                                     agb_align((size_t)ng * 4 * sizeof(GemmProb)));
-  ContractProb none = {};
-  prof_mark(AGB_ST_CONTRACT, s);
-  launch_contract<CX>(cp, none, maxL, maxR, ng, s);
-  AGB_CHECK_LAUNCH();
   const int maxm = 2 * maxL, maxn = 2 * maxR;
+  const int guard = (flags & AGB_RUN_NO_GUARD) ? 0 : 1;
   GemmCtx ctx;
   ctx.tc_bytes = tc_bytes;
   ctx.tc_scratch = tc_bytes ? ws + ws_bytes - tc_bytes : nullptr;
   ctx.status = status_word(ws, ng);
-  prof_mark(AGB_ST_GRAM, s);
-  int rc = launch_gemm_probs<CX>(gp + 2 * ng, ng, maxn, maxn, s, &ctx, maxm);
-  if (rc) return rc;
-  rc = launch_heevd_values<CX>(hp, ng, maxn, maxell, s);
-  if (rc) return rc;
-  prerank_kernel<CX><<<ng, 512, 0, s>>>(desc, ng, ws);
-  AGB_CHECK_LAUNCH();
-  rc = launch_heevd_vectors<CX>(hp, gp, ng, maxn, maxell, s, &ctx);
-  if (rc) return rc;
-  prof_mark(AGB_ST_AV, s);
-  rc = launch_gemm_probs<CX>(gp + 3 * ng, ng, maxm, maxell, s, &ctx, maxn);
-  if (rc) return rc;
-  prof_mark(AGB_ST_RANK, s);
-  const int guard = (flags & AGB_RUN_NO_GUARD) ? 0 : 1;
-  rank_kernel<CX><<<ng, 1024, 4 * (size_t)maxell * sizeof(double), s>>>(desc, ng, ws,
-                                                                          (flags & AGB_RUN_REPAIR) ? 0 : 2, guard);
-  AGB_CHECK_LAUNCH();
-  if (!(flags & AGB_RUN_REPAIR)) {
-    prof_mark(AGB_ST_GAP, s);
-    return AGB_OK;
+  int rc;
+  if (!(flags & AGB_RUN_REPAIR_ONLY)) {
+    if (cudaMemsetAsync(status_word(ws, ng), 0, sizeof(int), s) != cudaSuccess) return AGB_ERR_CUDA;
+    prof_mark(AGB_ST_SETUP, s);
+    setup_kernel<<<(ng + 127) / 128, 128, 0, s>>>(desc, ng, ws, esz);
+    AGB_CHECK_LAUNCH();
+    ContractProb* cp = (ContractProb*)(ws + agb_align((size_t)ng * sizeof(HeevdProb)) +
+                                       agb_align((size_t)ng * 4 * sizeof(GemmProb)));
+    ContractProb none = {};
+    prof_mark(AGB_ST_CONTRACT, s);
+    launch_contract<CX>(cp, none, maxL, maxR, ng, s);
+    AGB_CHECK_LAUNCH();
+    prof_mark(AGB_ST_GRAM, s);
+    rc = launch_gemm_probs<CX>(gp + 2 * ng, ng, maxn, maxn, s, &ctx, maxm);
+    if (rc) return rc;
+    rc = launch_heevd_values<CX>(hp, ng, maxn, maxell, s);
+    if (rc) return rc;
+    prerank_kernel<CX><<<ng, 512, 0, s>>>(desc, ng, ws);
+    AGB_CHECK_LAUNCH();
+    rc = launch_heevd_vectors<CX>(hp, gp, ng, maxn, maxell, s, &ctx);
+    if (rc) return rc;
+    prof_mark(AGB_ST_AV, s);
+    rc = launch_gemm_probs<CX>(gp + 3 * ng, ng, maxm, maxell, s, &ctx, maxn);
+    if (rc) return rc;
+    prof_mark(AGB_ST_RANK, s);
+    const int pass = (flags & (AGB_RUN_REPAIR | AGB_RUN_REPAIR_LATER)) ? 0 : 2;
+    rank_kernel<CX><<<ng, 1024, 4 * (size_t)maxell * sizeof(double), s>>>(desc, ng, ws, pass, guard);
+    AGB_CHECK_LAUNCH();
+    if (!(flags & AGB_RUN_REPAIR)) {
+      prof_mark(AGB_ST_GAP, s);
+      return AGB_OK;
+    }
   }
-  // repair pass for gates whose guided eigenvector count was too small
+  // repair pass for gates whose guided eigenvector count was too small: some 20
+  // launches, idle for nearly every batch (60-90 us of it), which a caller that
+  // reads the results back leaves out with AGB_RUN_REPAIR_LATER
   repair_setup_kernel<<<(ng + 127) / 128, 128, 0, s>>>(desc, ng, ws, guard);
   AGB_CHECK_LAUNCH();
   rc = launch_heevd_vectors<CX>(hp, gp, ng, maxn, maxell, s, &ctx);

@@ -124,6 +124,11 @@ int agb_two_site_plan(int dtype, int ngates, int64_t* desc_host, size_t* ws_byte
                           * without it such gates report AGB_ERR_RANK / AGB_ERR_NOCONV */
 #define AGB_RUN_NO_GUARD 2 /* flags: measure the orthogonality guard (AGB_D_ORTH/ORTHW) but
                             * neither repair nor reject on it */
+#define AGB_RUN_REPAIR_LATER 4 /* flags: leave those gates to a second call (below); a caller
+                                * that reads the results back anyway issues it only when some
+                                * gate reports AGB_ERR_RANK or an AGB_D_ORTH (AGB_D_MODE 0) above
+                                * 0.3 squared */
+#define AGB_RUN_REPAIR_ONLY 8 /* flags: that second call, on the same descriptors and workspace */
 int agb_two_site_run(int dtype, int ngates, const int64_t* desc_dev, int64_t* desc_dev_out,
                      int max_chiL, int max_chiM, int max_chiR, int max_ell, void* ws, size_t ws_bytes,
                      void* stream, int flags);
