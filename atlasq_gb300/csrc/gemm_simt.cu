@@ -1,7 +1,6 @@
-// SIMT batched complex GEMM for sm_103a, 256 threads.  complex64: 64 x 64 output
-// tiles, K-step 8, 4 x 4 complex accumulators per thread (small and ragged
-// shapes).  complex128: 16 x 16 tiles, K-step 16, one output per thread: the
-// FP64 pipe does 2 lanes per clock and SM whatever the tile, so what counts is
+// SIMT batched complex GEMM for sm_103a, 256 threads, K-step 16.  complex64:
+// 64 x 64 or 32 x 32 output tiles (launch_simt), for small and ragged shapes.
+// complex128: 16 x 16 tiles, one output per thread: the FP64 pipe does 2 lanes per clock and SM whatever the tile, so what counts is
 // how many SMs a product spreads over and how little of a ragged tile is
 // padding (a 10-gate layer at chi 48: 189 us over its 19 launches, 2043 us with
 // 64 x 64 tiles, 40 CTAs a launch and a third of their area padding).
@@ -9,10 +8,6 @@
 #include "gemm_tc.cuh"
 
 namespace {
-
-template <typename CX> struct Tile;
-template <> struct Tile<float2> { static constexpr int B = 64, K = 8, T = 4; };
-template <> struct Tile<double2> { static constexpr int B = 16, K = 16, T = 1; };
 
 template <typename CX>
 AGB_DEV CX load_op(const CX* P, int64_t ld, int op, int row, int col, int rows, int cols) {
@@ -41,16 +36,17 @@ AGB_DEV GemmProb get_prob(const GemmProb* probs, const StridedBatch& sb) {
   return p;
 }
 
-template <typename CX>
+// BT x BT tile, K-step BK, T x T outputs per thread (BT = 16 T).
+template <typename CX, int BT, int BK, int T>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restrict__ probs, StridedBatch sb,
                                                         int tiles_n) {
-  constexpr int BM = Tile<CX>::B, BN = Tile<CX>::B, BK = Tile<CX>::K, T = Tile<CX>::T;
+  constexpr int BM = BT, BN = BT;
   const GemmProb p = get_prob<CX>(probs, sb);
   const int m0 = (int)(blockIdx.x / tiles_n) * BM, n0 = (int)(blockIdx.x % tiles_n) * BN;
   if (m0 >= p.M || n0 >= p.N) return;
   typedef typename cx_traits<CX>::R R;
-  __shared__ CX As[BK][BM + 1];
-  __shared__ CX Bs[BK][BN + 1];
+  __shared__ CX As[2][BK][BM + 1];
+  __shared__ CX Bs[2][BK][BN + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const CX* A = (const CX*)p.A;
   const CX* B = (const CX*)p.B;
@@ -60,37 +56,52 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
 #pragma unroll
     for (int j = 0; j < T; ++j) acc[i][j] = czero<CX>();
 
-  for (int k0 = 0; k0 < p.K; k0 += BK) {
-    // A tile: BM x BK of op(A); B tile: BK x BN of op(B)
+  // A tile: BM x BK of op(A); B tile: BK x BN of op(B).  The next K step is read
+  // into registers while the current one is multiplied, and the two
+  // shared-memory buffers leave one barrier per step.
+  constexpr int NE = BM * BK / 256;
+  const bool an = p.opA == 0 || p.opA == 3, bn = p.opB == 0 || p.opB == 3;
+  CX va[NE], vb[NE];
+  auto fetch = [&](int k0) {
 #pragma unroll
-    for (int e = 0; e < BM * BK / 256; ++e) {
+    for (int e = 0; e < NE; ++e) {
       const int idx = tid + e * 256;
-      int r, c;
-      if (p.opA == 0 || p.opA == 3) { r = idx / BK; c = idx % BK; } else { r = idx % BM; c = idx / BM; }
-      As[c][r] = load_op(A, p.lda, p.opA, m0 + r, k0 + c, p.M, p.K);
-      int kr, nc;
-      if (p.opB == 0 || p.opB == 3) { kr = idx / BN; nc = idx % BN; } else { kr = idx % BK; nc = idx / BK; }
-      Bs[kr][nc] = load_op(B, p.ldb, p.opB, k0 + kr, n0 + nc, p.K, p.N);
+      const int r = an ? idx / BK : idx % BM, c = an ? idx % BK : idx / BM;
+      va[e] = load_op(A, p.lda, p.opA, m0 + r, k0 + c, p.M, p.K);
+      const int kr = bn ? idx / BN : idx % BK, nc = bn ? idx % BN : idx / BK;
+      vb[e] = load_op(B, p.ldb, p.opB, k0 + kr, n0 + nc, p.K, p.N);
+    }
+  };
+  fetch(0);
+  int buf = 0;
+  for (int k0 = 0; k0 < p.K; k0 += BK, buf ^= 1) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int idx = tid + e * 256;
+      const int r = an ? idx / BK : idx % BM, c = an ? idx % BK : idx / BM;
+      As[buf][c][r] = va[e];
+      const int kr = bn ? idx / BN : idx % BK, nc = bn ? idx % BN : idx / BK;
+      Bs[buf][kr][nc] = vb[e];
     }
     __syncthreads();
+    if (k0 + BK < p.K) fetch(k0 + BK);
     const int kn = min(BK, p.K - k0);
     if (T == 1 && kn < BK) {  // no padding products on the FP64 pipe
-      for (int k = 0; k < kn; ++k) cfma(acc[0][0], As[k][ty], Bs[k][tx]);
+      for (int k = 0; k < kn; ++k) cfma(acc[0][0], As[buf][k][ty], Bs[buf][k][tx]);
     } else {
 #pragma unroll
       for (int k = 0; k < BK; ++k) {
         CX a[T], b[T];
 #pragma unroll
-        for (int i = 0; i < T; ++i) a[i] = As[k][ty + 16 * i];
+        for (int i = 0; i < T; ++i) a[i] = As[buf][k][ty + 16 * i];
 #pragma unroll
-        for (int j = 0; j < T; ++j) b[j] = Bs[k][tx + 16 * j];
+        for (int j = 0; j < T; ++j) b[j] = Bs[buf][k][tx + 16 * j];
 #pragma unroll
         for (int i = 0; i < T; ++i)
 #pragma unroll
           for (int j = 0; j < T; ++j) cfma(acc[i][j], a[i], b[j]);
       }
     }
-    __syncthreads();
   }
   const CX alpha = mk<CX>((R)p.alpha_re, (R)p.alpha_im);
   const CX beta = mk<CX>((R)p.beta_re, (R)p.beta_im);
@@ -115,6 +126,29 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
 
 }  // namespace
 
+// complex64: 64 x 64 tiles where they give every SM one, else 32 x 32 (a 256 x
+// 512 x 256 product: 32 CTAs of 64 x 64 take 40 us, 128 of 32 x 32 23; five
+// 200 x 400 x 200: 33 against 31; but 16384 x 64 x 16: 6.9 against 8.2).  With one
+// tile size, K-step 8 and no read-ahead: 55, 44 and 7.2 us.
+template <typename CX>
+static int launch_simt(const GemmProb* probs, const StridedBatch& sb, int count, int64_t M, int64_t N,
+                       cudaStream_t s) {
+  auto tiles = [&](int b) { return ((N + b - 1) / b) * ((M + b - 1) / b); };
+  int b = 16;
+  if (sizeof(CX) == 8) b = tiles(64) * count >= 152 ? 64 : 32;
+  const int64_t t = tiles(b), tn = (N + b - 1) / b;
+  if (t > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)t, 1, count);
+  if constexpr (sizeof(CX) == 16) {
+    gemm_simt_kernel<CX, 16, 16, 1><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+  } else {
+    if (b == 64) gemm_simt_kernel<CX, 64, 16, 4><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    else gemm_simt_kernel<CX, 32, 16, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+  }
+  AGB_CHECK_LAUNCH();
+  return AGB_OK;
+}
+
 template <typename CX>
 int launch_gemm_probs(const GemmProb* probs, int count, int maxM, int maxN, cudaStream_t s, const GemmCtx* ctx,
                       int maxK) {
@@ -122,13 +156,7 @@ int launch_gemm_probs(const GemmProb* probs, int count, int maxM, int maxN, cuda
   if (sizeof(CX) == 8 && ctx && ctx->tc_scratch && maxM >= 64 && maxN >= 64 && maxK >= 32 &&
       ctx->tc_bytes >= tc_gemm_scratch_bytes(count, maxM, maxN, maxK))
     return launch_gemm_tc(probs, count, maxM, maxN, maxK, ctx->tc_scratch, ctx->tc_bytes, ctx->status, s);
-  constexpr int B = Tile<CX>::B;
-  const int tn = (maxN + B - 1) / B, tm = (maxM + B - 1) / B;
-  if ((int64_t)tn * tm > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
-  StridedBatch sb = {};
-  gemm_simt_kernel<CX><<<dim3(tn * tm, 1, count), 256, 0, s>>>(probs, sb, tn);
-  AGB_CHECK_LAUNCH();
-  return AGB_OK;
+  return launch_simt<CX>(probs, StridedBatch{}, count, maxM, maxN, s);
 }
 
 template int launch_gemm_probs<float2>(const GemmProb*, int, int, int, cudaStream_t, const GemmCtx*, int);
@@ -177,14 +205,6 @@ extern "C" int agb_cgemm_batched(int dtype, char opA, char opB, int batch, int M
   sb.sB = strideB;
   sb.sC = strideC;
   cudaStream_t s = (cudaStream_t)stream;
-  const int B_ = dtype == AGB_C64 ? Tile<float2>::B : Tile<double2>::B;
-  const int64_t tn = ((int64_t)N + B_ - 1) / B_, tm = ((int64_t)M + B_ - 1) / B_;
-  if (tn * tm > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
-  const dim3 grid((unsigned)(tn * tm), 1, batch);
-  if (dtype == AGB_C64)
-    gemm_simt_kernel<float2><<<grid, 256, 0, s>>>(nullptr, sb, (int)tn);
-  else
-    gemm_simt_kernel<double2><<<grid, 256, 0, s>>>(nullptr, sb, (int)tn);
-  AGB_CHECK_LAUNCH();
-  return AGB_OK;
+  return dtype == AGB_C64 ? launch_simt<float2>(nullptr, sb, batch, M, N, s)
+                          : launch_simt<double2>(nullptr, sb, batch, M, N, s);
 }

@@ -1,6 +1,7 @@
 """Tile edges of the SIMT kernels that choose a tile by type or size: the gate
 contraction (8 x 8 tiles for complex128, 16 x 16 and, for large grids, 32 x 32 for
-complex64) and the complex128 GEMM (16 x 16, K-step 16).  Against 64-bit (or
+complex64), the complex128 GEMM (16 x 16, K-step 16) and the complex64 one (64 x
+64 for large grids, else 32 x 32).  Against 64-bit (or
 wider than 64-bit for complex128: componentwise bound) references: a sum of K
 products in the working precision is within 2 K u of the sum of magnitudes
 (two multiply-adds per real product pair), plus 8 u for the 4 x 4 gate."""
@@ -38,13 +39,15 @@ def test_contract_gate_tiles(L, M, R, dt):
     assert bool(((got - ref).abs() <= 2 * (2 * M + 8) * unit * mag).all())
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 17, 16), (16, 16, 15), (33, 31, 47), (70, 96, 96)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 17, 16), (16, 16, 15), (33, 31, 47), (70, 96, 96), (65, 9700, 17),
+                                   (20000, 33, 31)])
 @pytest.mark.parametrize("opA,opB", [("N", "N"), ("C", "T"), ("R", "C")])
-def test_complex128_gemm_tiles(M, N, K, opA, opB):
+@pytest.mark.parametrize("dt", [torch.complex64, torch.complex128])
+def test_gemm_tiles(M, N, K, opA, opB, dt):
     g = torch.Generator().manual_seed(M + N + K)
-    A, B = _c((M, K) if opA in "NR" else (K, M), g), _c((K, N) if opB in "NR" else (N, K), g)
+    A, B = _c((M, K) if opA in "NR" else (K, M), g).to(dt), _c((K, N) if opB in "NR" else (N, K), g).to(dt)
     f = {"N": lambda x: x, "T": lambda x: x.T, "C": lambda x: x.mH, "R": lambda x: x.conj()}
-    got = ops.cgemm(A.to(DEV), B.to(DEV), opA, opB).cpu()
-    ref = f[opA](A) @ f[opB](B)
-    mag = f[opA](A).abs() @ f[opB](B).abs()
-    assert bool(((got - ref).abs() <= 2 * 2 * K * 2.0 ** -53 * mag).all())
+    got = ops.cgemm(A.to(DEV), B.to(DEV), opA, opB).cpu().to(torch.complex128)
+    a, b = f[opA](A.to(torch.complex128)), f[opB](B.to(torch.complex128))
+    unit = 2.0 ** -24 if dt == torch.complex64 else 2.0 ** -53
+    assert bool(((got - a @ b).abs() <= 2 * 2 * K * unit * (a.abs() @ b.abs())).all())
