@@ -10,10 +10,12 @@
 //   memory.
 // * Panel p is factored by its owner alone: warp w holds panel column w; per
 //   column the owner warp forms the reflector and one block barrier publishes
-//   it to the warps that apply it to their columns.  The owner then forms the
-//   triangular factor T_p of H_pb ... H_pb+QB-1 = I - V T V^H (forward,
-//   columnwise) and writes V_p (explicit zeros above the unit diagonal) and
-//   T_p to global memory (L2).
+//   it.  The later warps apply it to their columns; the earlier ones, whose
+//   columns are done, form its products with their reflectors, from which warp
+//   0 builds the next column of the triangular factor T_p of H_pb ... H_pb+QB-1 =
+//   I - V T V^H (forward, columnwise) one column behind; and the whole CTA
+//   writes it to global memory (L2; explicit zeros above the unit diagonal).
+//   When the last column is done, V_p and T_p are complete.
 // * One cluster barrier per panel; every CTA then applies Q_p^H = I - V T^H V^H
 //   to its later panels from a shared-memory copy of V_p:
 //   W = V^H Y, W = T^H W, Y -= V W.
@@ -22,9 +24,16 @@
 //
 // One cluster barrier per QB columns (the unblocked cluster kernel needs two
 // per column), and the trailing updates are QB-wide instead of rank-1.
+//
+// What bounds it: the chain owner's panel -> barrier -> next owner's update -> its
+// panel, on one SM at a time: the panel is a chain of QB columns (norm, reflector,
+// barrier, product, update), the update of QB columns by QB reflectors is bound by
+// that SM's FP32 pipe (2 QB^2 M complex multiply-adds).
+// 512 x 256 on 16 CTAs: 0.62 ms (0.99 before): panels 24 us, updates 7.5, the
+// thin Q 6 us a panel.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "householder.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -40,7 +49,7 @@ template <> struct QrbCfg<double2> { static constexpr int QB = 8; };
 
 struct QrbLayout {
   int QB, C, P, PF, npo, ld;
-  size_t panels, vloc, w, w2, t, vb, total;  // byte offsets
+  size_t panels, vloc, vloc2, w, w2, t, vb, total;  // byte offsets (vloc2 == vloc: one buffer of V)
 };
 
 AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C) {
@@ -55,10 +64,16 @@ AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C) {
   size_t o = 0;
   L.panels = o; o += (size_t)L.npo * QB * L.ld * esz;
   L.vloc = o;   o += (size_t)QB * L.ld * esz;
+  L.vloc2 = L.vloc;
   L.w = o;      o += (size_t)QB * L.npo * QB * esz;
   L.w2 = o;     o += (size_t)QB * L.npo * QB * esz;
   L.t = o;      o += (size_t)QB * QB * esz;
   L.vb = o;     o += (size_t)2 * M * esz;
+  // a second V buffer where it fits: the thin Q's panels are then read ahead
+  if (o + (size_t)QB * L.ld * esz <= kQrbSmemBudget) {
+    L.vloc2 = o;
+    o += (size_t)QB * L.ld * esz;
+  }
   L.total = o;
   return L;
 }
@@ -68,9 +83,9 @@ AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C) {
 // V (QB columns, stride ld, rows r0..M-1 valid) and T are in shared memory;
 // QB and ncol are multiples of 4.  Register tiles of 4 x 4 keep the
 // shared-memory traffic at two loads per four complex FMAs.
-template <typename CX>
+template <typename CX, int QB>
 AGB_DEV void qrb_apply(CX* Y, const int* ycols, int ncol, const CX* V, const CX* T, CX* W, CX* W2, int r0, int M,
-                       int ld, int QB, bool herm) {
+                       int ld, bool herm) {
   typedef typename cx_traits<CX>::R Rt;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr int NW = QBT / 32;
@@ -125,11 +140,13 @@ AGB_DEV void qrb_apply(CX* Y, const int* ycols, int ncol, const CX* V, const CX*
   // W2 = op(T) W   (T upper triangular)
   for (int pr = tid; pr < QB * ncol; pr += QBT) {
     const int i = pr / ncol, y = pr % ncol;
-    CX acc = czero<CX>();
+    CX acc = czero<CX>();  // T's other triangle is stored as zeros: no bound on k
     if (herm) {
-      for (int k = 0; k <= i; ++k) cfmac(acc, T[k * QB + i], W[k * ncol + y]);  // conj(T[k][i]) W[k][y]
+#pragma unroll
+      for (int k = 0; k < QB; ++k) cfmac(acc, T[k * QB + i], W[k * ncol + y]);  // conj(T[k][i]) W[k][y]
     } else {
-      for (int k = i; k < QB; ++k) cfma(acc, T[i * QB + k], W[k * ncol + y]);
+#pragma unroll
+      for (int k = 0; k < QB; ++k) cfma(acc, T[i * QB + k], W[k * ncol + y]);
     }
     W2[pr] = acc;
   }
@@ -144,6 +161,7 @@ AGB_DEV void qrb_apply(CX* Y, const int* ycols, int ncol, const CX* V, const CX*
     for (int jr = 0; jr < 4; ++jr)
 #pragma unroll
       for (int jc = 0; jc < 4; ++jc) acc[jr][jc] = czero<CX>();
+#pragma unroll 4
     for (int i = 0; i < QB; ++i) {
       CX v[4], w[4];
 #pragma unroll
@@ -186,6 +204,7 @@ __global__ void __launch_bounds__(QBT, 1)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CX* pan = (CX*)(smem_raw + Lo.panels);  // own panels: local column s * QB + jj
   CX* Vl = (CX*)(smem_raw + Lo.vloc);
+  CX* V2 = (CX*)(smem_raw + Lo.vloc2);
   CX* W = (CX*)(smem_raw + Lo.w);
   CX* W2 = (CX*)(smem_raw + Lo.w2);
   CX* Tl = (CX*)(smem_raw + Lo.t);
@@ -193,7 +212,8 @@ __global__ void __launch_bounds__(QBT, 1)
   __shared__ int ycols[kQrbMaxCols];
   __shared__ int ycount;
   __shared__ CX taus[QB];
-  __shared__ CX Ssh[QB * QB];
+  constexpr int TP = QB + 1;
+  __shared__ CX Ssh[QB * TP], Tsh[QB * TP];
   // own panels: p = q + s * C
   const int nown = (q < Lo.P) ? (Lo.P - q + C - 1) / C : 0;
   // ---- load own columns of op(A)
@@ -230,71 +250,76 @@ __global__ void __launch_bounds__(QBT, 1)
           x[k] = (r < M) ? col[r] : czero<CX>();
         }
       }
+      CX* Vp = Vg + (size_t)p * QB * M;
+      // T[k][i] = -tau_i sum_{k <= m < i} T[k][m] S[m][i] (lane k of warp 0), T[i][i] = tau_i
+      auto t_column = [&](int i) {
+        if (lane < i) {
+          CX acc = czero<CX>();
+          for (int m = lane; m < i; ++m) cfma(acc, Tsh[lane * TP + m], Ssh[m * TP + i]);
+          const CX ti = taus[i];
+          Tsh[lane * TP + i] = cmul(mk<CX>(-ti.x, -ti.y), acc);
+        } else if (lane < QB) {
+          Tsh[lane * TP + i] = lane == i ? taus[i] : czero<CX>();
+        }
+        __syncwarp();
+      };
       for (int jj = 0; jj < bw; ++jj) {
         const int c = pb + jj;
         CX* vb = vbuf + (size_t)(jj & 1) * M;
         if (wid == jj) {
-          Rt part = 0;
+          Rt p0 = 0, p1 = 0;
           CX am = czero<CX>();
 #pragma unroll
           for (int k = 0; k < NK; ++k) {
             const int r = lane + 32 * k;
-            if (r > c && r < M) part += cabs2(x[k]);
+            const Rt z = cabs2(x[k]);  // rows past M hold zeros
+            if (k & 1) p1 += r > c ? z : Rt(0);
+            else p0 += r > c ? z : Rt(0);
             if (r == c) am = x[k];
           }
-          const Rt xn2 = warp_sum(part);
+          const Rt xn2 = warp_sum(p0 + p1);
           CX alpha;
           alpha.x = __shfl_sync(0xffffffffu, am.x, c & 31);
           alpha.y = __shfl_sync(0xffffffffu, am.y, c & 31);
-          CX t = czero<CX>(), sc = czero<CX>();
+          CX t, sc;
           Rt beta;
-          if (xn2 == Rt(0) && alpha.y == Rt(0)) {
-            beta = alpha.x;
-          } else {
-            beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-            t = mk<CX>((beta - alpha.x) / beta, -alpha.y / beta);
-            sc = cinv(csub(alpha, mk<CX>(beta, 0)));
-          }
+          reflector(alpha, xn2, beta, t, sc);
 #pragma unroll
           for (int k = 0; k < NK; ++k) {
             const int r = lane + 32 * k;
-            if (r < M) {
-              CX v = czero<CX>();
-              if (r == c) {
-                v = mk<CX>(1, 0);
-                x[k] = mk<CX>(beta, 0);
-              } else if (r > c) {
-                x[k] = cmul(x[k], sc);  // v below the diagonal
-                v = x[k];
-              }
-              vb[r] = v;
-            }
+            const CX u = cmul(x[k], sc);
+            const CX v = r > c ? u : r == c ? mk<CX>(1, 0) : czero<CX>();
+            if (r < M) vb[r] = v;
+            x[k] = r > c ? u : r == c ? mk<CX>(beta, 0) : x[k];  // v below the diagonal
           }
           if (lane == 0) taus[jj] = t;
         }
         __syncthreads();
-        // H_c^H = I - conj(tau) v v^H on the panel's later columns
-        if (wid > jj && wid < pw) {
-          const CX t = taus[jj];
-          if (t.x != Rt(0) || t.y != Rt(0)) {
-            CX a0 = czero<CX>(), a1 = czero<CX>();
+        // v_c^H x: for the later columns H_c^H = I - conj(tau) v v^H is applied, for
+        // the earlier ones (x = v_w below its diagonal) it is conj(S[w][jj])
+        if (wid != jj && wid < pw) {
+          CX a0 = czero<CX>(), a1 = czero<CX>();
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            const int r = lane + 32 * k;
+            const CX vr = r < M ? vb[r] : czero<CX>();  // zero above row c
+            if (k & 1) cfmac(a1, vr, x[k]);
+            else cfmac(a0, vr, x[k]);
+          }
+          const CX acc = warp_csum(cadd(a0, a1));
+          if (wid > jj) {
+            const CX tw = cmul(cconj(taus[jj]), acc);
 #pragma unroll
             for (int k = 0; k < NK; ++k) {
               const int r = lane + 32 * k;
-              if (r >= c && r < M) {
-                if (k & 1) cfmac(a1, vb[r], x[k]);
-                else cfmac(a0, vb[r], x[k]);
-              }
+              if (r < M) x[k] = csub(x[k], cmul(vb[r], tw));
             }
-            const CX acc = warp_csum(cadd(a0, a1));
-            const CX tw = cmul(cconj(t), acc);
-#pragma unroll
-            for (int k = 0; k < NK; ++k) {
-              const int r = lane + 32 * k;
-              if (r >= c && r < M) x[k] = csub(x[k], cmul(vb[r], tw));
-            }
+          } else if (lane == 0) {
+            Ssh[wid * TP + jj] = cconj(acc);
           }
         }
+        for (int r = tid; r < M; r += QBT) Vp[(size_t)jj * M + r] = vb[r];
+        if (wid == 0 && jj > 0) t_column(jj - 1);  // S[.][jj-1] is complete since the barrier
       }
       if (wid < pw) {
         CX* col = P0 + (size_t)wid * ld;
@@ -305,53 +330,13 @@ __global__ void __launch_bounds__(QBT, 1)
         }
       }
       __syncthreads();
-      // V_p to global (explicit zeros above the unit diagonal; zero columns past bw)
-      CX* Vp = Vg + (size_t)p * QB * M;
-      for (int idx = tid; idx < QB * M; idx += QBT) {
-        const int jj = idx / M, r = idx % M;
-        const int c = pb + jj;
-        CX v = czero<CX>();
-        if (jj < bw) v = (r < c) ? czero<CX>() : (r == c ? mk<CX>(1, 0) : P0[(size_t)jj * ld + r]);
-        Vp[idx] = v;
-      }
-      // S[k][i] = v_k^H v_i (k < i), pairs round-robin over the warps
-      for (int pr = wid; pr < QB * QB; pr += QBT / 32) {
-        const int k = pr / QB, i = pr % QB;
-        if (k < i && i < bw) {
-          const CX* vk = P0 + (size_t)k * ld;
-          const CX* vi = P0 + (size_t)i * ld;
-          const int ci = pb + i;
-          CX acc = czero<CX>();
-          for (int r = ci + lane; r < M; r += 32)
-            cfmac(acc, vk[r], (r == ci) ? mk<CX>(1, 0) : vi[r]);  // v_k[ci] is below v_k's diagonal
-          acc = warp_csum(acc);
-          if (lane == 0) Ssh[pr] = acc;
-        }
-      }
-      __syncthreads();
-      // T (forward, columnwise): T[i][i] = tau_i, T[0:i][i] = -tau_i T[0:i][0:i] S[0:i][i];
-      // lane k of warp 0 holds row k of T in registers
       if (wid == 0) {
-        CX trow[QB];
-#pragma unroll
-        for (int m = 0; m < QB; ++m) trow[m] = czero<CX>();
-#pragma unroll
-        for (int i = 0; i < QB; ++i) {
-          if (i < bw) {
-            const CX ti = taus[i];
-            CX acc = czero<CX>();
-#pragma unroll
-            for (int m = 0; m < i; ++m)
-              if (m >= lane) cfma(acc, trow[m], Ssh[m * QB + i]);
-            if (lane < i) trow[i] = cmul(mk<CX>(-ti.x, -ti.y), acc);
-            else if (lane == i) trow[i] = ti;
-          }
-        }
+        if (bw > 0) t_column(bw - 1);
         CX* Tp = Tg + (size_t)p * QB * QB;
-        if (lane < QB)
-#pragma unroll
-          for (int m = 0; m < QB; ++m) Tp[lane * QB + m] = trow[m];
+        for (int e = lane; e < QB * QB; e += 32)
+          Tp[e] = e % QB < bw && e / QB < bw ? Tsh[(e / QB) * TP + e % QB] : czero<CX>();
       }
+      for (int e = tid; e < (QB - bw) * M; e += QBT) Vp[(size_t)bw * M + e] = czero<CX>();  // past bw
       __threadfence();  // V_p, T_p visible to the cluster before the barrier
     }
     cluster.sync();
@@ -369,13 +354,13 @@ __global__ void __launch_bounds__(QBT, 1)
     const int ncol = ycount;
     if (ncol > 0) {
       const CX* Vp = Vg + (size_t)p * QB * M;
-      for (int idx = tid; idx < QB * (M - pb); idx += QBT) {
-        const int jj = idx / (M - pb), r = pb + idx % (M - pb);
-        Vl[(size_t)jj * ld + r] = __ldcg(Vp + (size_t)jj * M + r);
+      for (int jj = wid; jj < QB; jj += QBT / 32) {
+#pragma unroll 8
+        for (int r = pb + lane; r < M; r += 32) Vl[(size_t)jj * ld + r] = __ldcg(Vp + (size_t)jj * M + r);
       }
       for (int e = tid; e < QB * QB; e += QBT) Tl[e] = __ldcg(Tg + (size_t)p * QB * QB + e);
       __syncthreads();
-      qrb_apply(pan, ycols, ncol, Vl, Tl, W, W2, pb, M, ld, QB, true);
+      qrb_apply<CX, QB>(pan, ycols, ncol, Vl, Tl, W, W2, pb, M, ld, true);
     }
   }
   // ---- R = upper triangle of the factored columns (kk x N)
@@ -393,55 +378,62 @@ __global__ void __launch_bounds__(QBT, 1)
     }
   }
   __syncthreads();
-  // ---- thin Q: own columns c < kk, Z = [I; 0] in the panel storage, Z <- Q_p Z backwards
-  for (int s = 0; s < nown; ++s) {
-    const int p = q + s * C;
-    for (int jj = wid; jj < QB; jj += QBT / 32) {
-      const int c = p * QB + jj;
-      CX* col = pan + (size_t)(s * QB + jj) * ld;
-      for (int r = lane; r < M; r += 32) col[r] = (r == c && c < kk) ? mk<CX>(1, 0) : czero<CX>();
-    }
+  // ---- thin Q: Z = [I; 0] in the panel storage, Z <- Q_p Z backwards.  The columns
+  // are dealt to the CTAs one by one (column q + m C in slot m), so that each
+  // panel's work, on the columns from its first on, is spread evenly: by panels,
+  // the last CTA had every panel to apply to all its columns.
+  const int nq = q < kk ? (kk - q + C - 1) / C : 0;      // own columns of Q
+  const int nq4 = (nq + 3) & ~3;                    // slots in use (the update takes fours) <= npo QB
+  for (int m = wid; m < nq4; m += QBT / 32) {
+    const int c = m < nq ? q + m * C : -1;
+    CX* col = pan + (size_t)m * ld;
+    for (int r = lane; r < M; r += 32) col[r] = (r == c) ? mk<CX>(1, 0) : czero<CX>();
   }
   __syncthreads();
-  for (int p = Lo.PF - 1; p >= 0; --p) {
+  // V_p to buffer buf by asynchronous copies (its rows >= pb), T_p with it
+  auto read_panel = [&](int p, CX* Vd) {
     const int pb = p * QB;
-    if (tid == 0) {
-      int nc = 0;
-      for (int s = 0; s < nown; ++s) {
-        const int pp = q + s * C;
-        if (pp >= p && pp < Lo.PF)  // columns c < pb are e_c, untouched by Q_p
-          for (int jj = 0; jj < QB; ++jj) ycols[nc++] = s * QB + jj;
-      }
-      ycount = nc;
-    }
-    __syncthreads();
-    const int ncol = ycount;
-    if (ncol == 0) continue;
     const CX* Vp = Vg + (size_t)p * QB * M;
-    for (int idx = tid; idx < QB * (M - pb); idx += QBT) {
-      const int jj = idx / (M - pb), r = pb + idx % (M - pb);
-      Vl[(size_t)jj * ld + r] = __ldcg(Vp + (size_t)jj * M + r);
-    }
+    for (int jj = wid; jj < QB; jj += QBT / 32)
+      for (int r = pb + lane; r < M; r += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(Vd + (size_t)jj * ld + r)),
+                     "l"(Vp + (size_t)jj * M + r), "n"((int)sizeof(CX))
+                     : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const bool ahead = Lo.vloc2 != Lo.vloc;
+  const int plast = nq4 > 0 ? Lo.PF - 1 : -1;
+  if (ahead && plast >= 0) read_panel(plast, Vl);
+  for (int p = plast; p >= 0; --p) {
+    const int pb = p * QB;
+    // slots of the columns >= pb (columns below pb are e_c, which Q_p leaves alone)
+    const int m0 = (pb > q ? (pb - q + C - 1) / C : 0) & ~3;
+    const int ncol = nq4 > m0 ? nq4 - m0 : 0;
+    for (int m = tid; m < ncol; m += QBT) ycols[m] = m0 + m;
+    CX* Vd = ahead && ((plast - p) & 1) ? V2 : Vl;
     for (int e = tid; e < QB * QB; e += QBT) Tl[e] = __ldcg(Tg + (size_t)p * QB * QB + e);
+    if (!ahead) read_panel(p, Vd);
+    if (ahead && p > 0) {
+      read_panel(p - 1, Vd == Vl ? V2 : Vl);  // that buffer's panel was applied before the last barrier
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
-    qrb_apply(pan, ycols, ncol, Vl, Tl, W, W2, pb, M, ld, QB, false);
+    qrb_apply<CX, QB>(pan, ycols, ncol, Vd, Tl, W, W2, pb, M, ld, false);
+    if (ncol == 0) __syncthreads();  // the update's last barrier frees the buffers
   }
   // ---- write Q (M x kk, or its transpose)
-  for (int s = 0; s < nown; ++s) {
-    const int p = q + s * C;
-    if (trans_out) {
-      for (int jj = wid; jj < QB; jj += QBT / 32) {
-        const int c = p * QB + jj;
-        if (c >= kk) continue;
-        const CX* col = pan + (size_t)(s * QB + jj) * ld;
-        for (int r = lane; r < M; r += 32) Q[(int64_t)c * M + r] = col[r];
-      }
-    } else {
-      const int nc = min(QB, kk - p * QB);
-      for (int idx = tid; idx < M * (nc > 0 ? nc : 0); idx += QBT) {
-        const int r = idx / nc, jj = idx % nc;
-        Q[(int64_t)r * kk + p * QB + jj] = pan[(size_t)(s * QB + jj) * ld + r];
-      }
+  if (trans_out) {
+    for (int m = wid; m < nq; m += QBT / 32) {
+      const CX* col = pan + (size_t)m * ld;
+      for (int r = lane; r < M; r += 32) Q[(int64_t)(q + m * C) * M + r] = col[r];
+    }
+  } else {
+    for (int m = wid; m < nq; m += QBT / 32) {
+      const CX* col = pan + (size_t)m * ld;
+      for (int r = lane; r < M; r += 32) Q[(int64_t)r * kk + q + m * C] = col[r];
     }
   }
   cluster.sync();

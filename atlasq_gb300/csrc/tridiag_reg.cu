@@ -36,6 +36,7 @@
 // (real), tau, reflector v_j in row j of H (columns j+2 .., v_j[j+1] = 1
 // implicit), scale.
 #include "heevd.cuh"
+#include "householder.cuh"
 #include "prof.cuh"
 
 namespace {
@@ -86,27 +87,6 @@ AGB_DEV bool bar_wait(uint32_t bar, uint32_t parity) {
 AGB_DEV void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Reflector of (alpha, x) with ||x||^2 = xn2 (zlarfg): beta, tau and the factor
-// 1 / (alpha - beta) of x.  A column whose norm underflows is left as it is.
-AGB_DEV void reflector(float2 alpha, float xn2, float& beta, float2& t, float2& sc) {
-  const float ss = fmaf(alpha.x, alpha.x, fmaf(alpha.y, alpha.y, xn2));
-  if ((xn2 == 0.f && alpha.y == 0.f) || ss <= 1e-36f) {
-    beta = alpha.x;
-    t = sc = make_float2(0.f, 0.f);
-    return;
-  }
-  // 1 / sqrt(ss) with one Newton step, the norm from it
-  float y = rsqrtf(ss);
-  y = fmaf(0.5f * y, fmaf(-ss * y, y, 1.f), y);
-  const float m = ss * y;
-  beta = -copysignf(m, alpha.x);
-  const float ib = -copysignf(y, alpha.x);
-  t = make_float2((beta - alpha.x) * ib, -alpha.y * ib);
-  const float dx = alpha.x - beta;  // no cancellation: beta has the other sign
-  const float id = __frcp_rn(fmaf(dx, dx, alpha.y * alpha.y));
-  sc = make_float2(dx * id, -alpha.y * id);
 }
 
 // CTAs that reduce an n x n matrix in a launch of C-CTA clusters: a matrix whose
