@@ -82,6 +82,10 @@ _SIGS = {
     "agb_sample_site": (I, [I, P, I, I, I, U64, U64, P, P, P, P]),
     "agb_mpo_mix": (I, [I, P, P, P, I, I, I, I, P]),
     "agb_trace_prod": (I, [I, P, P, I, P, P]),
+    "agb_site_mix_list": (I, [I, P, I, I64, P]),
+    "agb_trace_prod_list": (I, [I, P, I, P, P]),
+    "agb_gemm_prob_bytes": (SZ, []),
+    "agb_gemm_list": (I, [I, I, P, I, I, I, I, P, P]),
     "agb_mpo_apply_site": (I, [I, P, P, P, I, I, I, I, P]),
     "agb_tdvp_local_h_workspace": (SZ, [I, I, I, I, I]),
     "agb_tdvp_local_h": (I, [I, P, P, P, P, P, I, I, I, I, I, I, P, SZ, P]),

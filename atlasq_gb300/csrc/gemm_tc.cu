@@ -546,6 +546,27 @@ int launch_gemm_tc(const GemmProb* probs, int count, int maxM, int maxN, int max
   return launch_tc(probs, none, count, maxM, maxN, maxK, scratch, scratch_bytes, status, s);
 }
 
+// Products listed in device memory, any shapes, one launch.
+extern "C" size_t agb_gemm_prob_bytes(void) { return sizeof(GemmProb); }
+
+extern "C" int agb_gemm_list(int dtype, int tensor_cores, const void* probs, int count, int maxM, int maxN, int maxK,
+                             int* status_dev, void* stream) {
+  if (dtype != AGB_C64 && dtype != AGB_C128) return AGB_ERR_ARG;
+  if (count < 0 || maxM < 0 || maxN < 0 || maxK < 0 || count > 65535) return AGB_ERR_ARG;
+  if (count == 0 || maxM == 0 || maxN == 0) return AGB_OK;
+  if (!probs) return AGB_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  const GemmProb* p = (const GemmProb*)probs;
+  if (tensor_cores) {
+    if (dtype != AGB_C64 || !status_dev) return AGB_ERR_ARG;
+    // the split operands live in shared memory: the scratch is a token
+    return launch_gemm_tc(p, count, maxM, maxN, maxK, status_dev, tc_gemm_scratch_bytes(count, maxM, maxN, maxK),
+                          status_dev, s);
+  }
+  return dtype == AGB_C64 ? launch_gemm_probs<float2>(p, count, maxM, maxN, s)
+                          : launch_gemm_probs<double2>(p, count, maxM, maxN, s);
+}
+
 // Strided-batch host entry for the tensor-core GEMM (complex64).
 namespace {
 int opc(char c) {

@@ -2,6 +2,7 @@
 current stream; every computation is a kernel of ``libatlasq_gb300.so``."""
 import ctypes
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -133,6 +134,57 @@ def single_qubit_gate_(T, U):
     check(lib.agb_single_qubit_gate(dtype_code(T.dtype), ptr(T), ptr(U), T.shape[0], T.shape[2],
                                     stream_ptr(T.device)), "single_qubit_gate")
     return T
+
+
+_PROB = np.dtype([("A", "u8"), ("B", "u8"), ("D", "u8"), ("C", "u8"), ("lda", "i8"), ("ldb", "i8"), ("ldd", "i8"),
+                  ("ldc", "i8"), ("M", "i4"), ("N", "i4"), ("K", "i4"), ("opA", "i4"), ("opB", "i4"), ("pad", "i4"),
+                  ("alpha_re", "f8"), ("alpha_im", "f8"), ("beta_re", "f8"), ("beta_im", "f8"), ("eye", "f8")])
+_OPC = {"N": 0, "T": 1, "C": 2, "R": 3}
+
+
+class ProductList:
+    """Products D = op(A) op(B) of any shapes: listed on the host in groups,
+    uploaded once, then launched group by group (one launch, or two where a
+    group has both kinds).  complex64 products with every dimension >= 32 take
+    the tcgen05 GEMM (3xTF32, float32 accuracy), the rest the SIMT GEMM."""
+
+    def __init__(self, dtype, device):
+        self.code, self.device = dtype_code(dtype), device
+        self.rows, self.groups = [], []
+        self.dev = None
+
+    def group(self, products):
+        """products: (M, N, K, opA, opB, A, lda, B, ldb, D, ldd) with device pointers; returns the group's number."""
+        tc = [p for p in products if self.code == _lib.AGB_C64 and min(p[0], p[1], p[2]) >= 32]
+        rest = [p for p in products if not (self.code == _lib.AGB_C64 and min(p[0], p[1], p[2]) >= 32)]
+        launches = []
+        for on, ps in ((1, tc), (0, rest)):
+            if ps:
+                launches.append((on, len(self.rows), len(ps), max(p[0] for p in ps), max(p[1] for p in ps),
+                                 max(p[2] for p in ps)))
+                self.rows += ps
+        self.groups.append(launches)
+        return len(self.groups) - 1
+
+    def upload(self):
+        assert _lib.load().agb_gemm_prob_bytes() == _PROB.itemsize
+        arr = np.zeros(len(self.rows), dtype=_PROB)
+        if self.rows:
+            num = np.array([(p[0], p[1], p[2], _OPC[p[3]], _OPC[p[4]]) + tuple(p[5:]) for p in self.rows],
+                           dtype=np.int64)
+            for k, name in enumerate(("M", "N", "K", "opA", "opB", "A", "lda", "B", "ldb", "D", "ldd")):
+                arr[name] = num[:, k]
+            arr["C"], arr["ldc"], arr["alpha_re"] = arr["D"], arr["ldd"], 1.0
+        self.dev = torch.from_numpy(arr.view(np.uint8)).to(self.device)
+        self.base, self.stream = self.dev.data_ptr(), stream_ptr(self.device)
+        self.status = ptr(_tc_status_word(self.device))
+        return self
+
+    def launch(self, g):
+        lib = _lib.load()
+        for on, first, count, M, N, K in self.groups[g]:
+            check(lib.agb_gemm_list(self.code, on, self.base + first * _PROB.itemsize, count, M, N, K, self.status,
+                                    self.stream), "gemm_list")
 
 
 _TC_STATUS = {}

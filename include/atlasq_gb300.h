@@ -251,6 +251,22 @@ int agb_tdvp_local_h(int dtype, const void* L, const void* W, const void* A, con
                      int Dl, int chiI, int Dn, int chiU, int chiJ, void* ws, size_t ws_bytes, void* stream);
 /* out2[0] + i out2[1] = sum_{r,c} E[r,c] Q[c,r]  (double accuracy; out2 is device memory). */
 int agb_trace_prod(int dtype, const void* E, const void* Q, int n, double* out2, void* stream);
+/* The same two operations for lists of items of any shapes, one launch each.
+ * agb_site_mix_list: items (device, int64) [count][5] = {M, W, N, chiA, chiB}, W one
+ * 2x2 operator; max_elems bounds chiA * chiB.  agb_trace_prod_list: items [count][3]
+ * = {E, Q, n}, out2 [count][2] double. */
+int agb_site_mix_list(int dtype, const int64_t* items, int count, int64_t max_elems, void* stream);
+int agb_trace_prod_list(int dtype, const int64_t* items, int count, double* out2, void* stream);
+/* Complex products D = alpha op(A) op(B) + beta C + eye I of any shapes in one launch:
+ * probs (device) holds `count` records of agb_gemm_prob_bytes() bytes:
+ *   const void *A, *B, *D, *C; int64 lda, ldb, ldd, ldc; int32 M, N, K, opA, opB, pad;
+ *   double alpha_re, alpha_im, beta_re, beta_im, eye      (op 0 N, 1 T, 2 C, 3 conj)
+ * with M, N, K bounded by maxM, maxN, maxK.  tensor_cores (complex64 only, K >= 1):
+ * the agb_cgemm_tc kernel, a wait that expires recorded in *status_dev; else
+ * the agb_cgemm_batched kernel (status_dev may be NULL). */
+size_t agb_gemm_prob_bytes(void);
+int agb_gemm_list(int dtype, int tensor_cores, const void* probs, int count, int maxM, int maxN, int maxK,
+                  int* status_dev, void* stream);
 
 /* Where the most recent failed launch check of this library was, as
  * "file:line: cudaErrorName (description)"; empty if none (this build's own
