@@ -12,6 +12,7 @@
 // is the projection of X onto the kept right singular subspace.
 #include <math.h>
 
+#include "eigvec.cuh"
 #include "gemm_tc.cuh"
 #include "heevd.cuh"
 #include "prof.cuh"
@@ -618,6 +619,8 @@ __global__ void __launch_bounds__(1024) rank_kernel(int64_t* __restrict__ desc, 
   D[AGB_D_ORTHW] = bitsd(mode0 == 1 ? 0.0 : (double)__uint_as_float(hp[g].orth_w2));
 }
 
+#include "small_gate.cuh"
+
 // ------------------------------------------------------------------ scatter
 template <typename CX>
 __global__ void scatter_kernel(const int64_t* __restrict__ desc, char* ws) {
@@ -751,6 +754,18 @@ int run_impl(int ng, int64_t* desc, int maxL, int maxM, int maxR, int maxell, ch
     if (rc) return rc;
     prerank_kernel<CX><<<ng, 512, 0, s>>>(desc, ng, ws);
     AGB_CHECK_LAUNCH();
+    if (sizeof(CX) == 8 && maxm <= kSmallMax && maxn <= kSmallMax && maxell <= kSmallMax &&
+        tridiag_stages_mode() == 1) {
+      // vectors, X V, rank selection and the repair of every gate in one launch
+      prof_mark(AGB_ST_INVIT, s);
+      const size_t sm = small_layout().total;
+      if (agb_smem_optin(small_gate_kernel, sm) != cudaSuccess) return AGB_ERR_CUDA;
+      small_gate_kernel<<<ng, kSmallThreads, sm, s>>>(
+          desc, ng, ws, guard, (flags & (AGB_RUN_REPAIR | AGB_RUN_REPAIR_LATER)) ? 1 : 0);
+      AGB_CHECK_LAUNCH();
+      prof_mark(AGB_ST_GAP, s);
+      return AGB_OK;
+    }
     rc = launch_heevd_vectors<CX>(hp, gp, ng, maxn, maxell, s, &ctx);
     if (rc) return rc;
     prof_mark(AGB_ST_AV, s);
