@@ -84,6 +84,7 @@ _SIGS = {
     "agb_trace_prod": (I, [I, P, P, I, P, P]),
     "agb_site_mix_list": (I, [I, P, I, I64, P]),
     "agb_trace_prod_list": (I, [I, P, I, P, P]),
+    "agb_statevector": (I, [I, I, P, P, P, P]),
     "agb_gemm_prob_bytes": (SZ, []),
     "agb_gemm_list": (I, [I, I, P, I, I, I, I, P, P]),
     "agb_mpo_apply_site": (I, [I, P, P, P, I, I, I, I, P]),

@@ -375,10 +375,12 @@ class AdaptiveMPS:
         if self.num_qubits > 20:
             raise ValueError(f"Converting {self.num_qubits} qubits to statevector would require "
                              f"{2**self.num_qubits} amplitudes. Use get_amplitude() for large systems.")
-        T = self.tensors
-        res = self._common(T[0]).reshape(2, -1)  # [2, chi1]
+        T = [self._common(t) for t in self.tensors]
+        psi = ops.statevector(T)
+        if psi is not None:
+            return psi
+        res = T[0].reshape(2, -1)  # [2, chi1]
         for t in T[1:]:
-            t = self._common(t)
             res = ops.cgemm(res.contiguous(), t.reshape(t.shape[0], -1)).reshape(-1, t.shape[2])
         return res.reshape(-1)
 

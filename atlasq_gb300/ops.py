@@ -142,6 +142,25 @@ _PROB = np.dtype([("A", "u8"), ("B", "u8"), ("D", "u8"), ("C", "u8"), ("lda", "i
 _OPC = {"N": 0, "T": 1, "C": 2, "R": 3}
 
 
+def statevector(tensors):
+    """Dense state of a short open chain (contiguous [chi_s, 2, chi_s+1] tensors of
+    one dtype and device) in one launch; None where the chain does not fit one."""
+    n = len(tensors)
+    t0 = tensors[0]
+    chi = [t.shape[0] for t in tensors] + [tensors[-1].shape[-1]]
+    if not 2 <= n <= 20 or min(chi) < 1 or chi[0] != 1 or chi[n] != 1 or any(
+            t.shape != (chi[s], 2, chi[s + 1]) or t.dtype != t0.dtype or t.device != t0.device
+            or not t.is_contiguous() or not t.is_cuda or t.is_conj() for s, t in enumerate(tensors)):
+        return None
+    out = torch.empty(1 << n, dtype=t0.dtype, device=t0.device)
+    rc = _lib.load().agb_statevector(dtype_code(t0.dtype), n, (ctypes.c_int64 * n)(*[t.data_ptr() for t in tensors]),
+                                     (ctypes.c_int32 * (n + 1))(*chi), ptr(out), stream_ptr(t0.device))
+    if rc == _lib.AGB_ERR_UNSUPPORTED:
+        return None
+    check(rc, "statevector")
+    return out
+
+
 class ProductList:
     """Products D = op(A) op(B) of any shapes: listed on the host in groups,
     uploaded once, then launched group by group (one launch, or two where a

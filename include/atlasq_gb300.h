@@ -257,6 +257,11 @@ int agb_trace_prod(int dtype, const void* E, const void* Q, int n, double* out2,
  * = {E, Q, n}, out2 [count][2] double. */
 int agb_site_mix_list(int dtype, const int64_t* items, int count, int64_t max_elems, void* stream);
 int agb_trace_prod_list(int dtype, const int64_t* items, int count, double* out2, void* stream);
+/* Dense state of an open chain of n sites in one launch: tensors[s] (host array of
+ * device pointers) is [chi[s], 2, chi[s+1]], chi[0] = chi[n] = 1; out has 2^n elements,
+ * site 0 the most significant qubit.  AGB_ERR_UNSUPPORTED (nothing launched) for chains
+ * too long or too wide for one launch. */
+int agb_statevector(int dtype, int n, const int64_t* tensors, const int32_t* chi, void* out, void* stream);
 /* Complex products D = alpha op(A) op(B) + beta C + eye I of any shapes in one launch:
  * probs (device) holds `count` records of agb_gemm_prob_bytes() bytes:
  *   const void *A, *B, *D, *C; int64 lda, ldb, ldd, ldc; int32 M, N, K, opA, opB, pad;
