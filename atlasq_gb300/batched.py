@@ -158,7 +158,7 @@ class CapturedCircuit:
                 # can be rewritten between replays (update_gates)
                 U2 = torch.stack([U.to(device=device, dtype=dt).reshape(4, 4) for _, _, U in twos]).contiguous()
                 staged = [(m, i, U2[g]) for g, (m, i, _) in enumerate(twos)]
-                desc, wsz, dims, keep = resident.build_two_site(staged)
+                desc, wsz, dims, keep, _, _ = resident.build_two_site(staged)
                 self.keep.append(keep)
                 step["twos"] = (torch.from_numpy(desc).to(device), wsz, dims, len(twos), staged)
                 step["U2"] = U2
@@ -276,8 +276,10 @@ class CapturedCircuit:
                 for k, rs in per.items():
                     rows.setdefault(k, []).append((d, rs, now))
         for m, (res, _, _) in zip(self.batch.instances, self.start):
-            m._pending, m._pending_1q, m._pending_sites = [], [], set()
             res.batches = rows.get(id(m), [])
+        back = resident.ReadBack([res for res, _, _ in self.start])
+        for m, (res, _, _) in zip(self.batch.instances, self.start):
+            m._pending, m._pending_1q, m._pending_sites = [], [], set()
             m._res = res
-            resident.leave(m)
+            resident.leave(m, back)
         return self.batch

@@ -53,17 +53,18 @@ class _PinnedRing:
         self.events = [None] * nslots
         self.next = 0
 
-    def upload(self, arr: np.ndarray) -> torch.Tensor:
+    def upload(self, arr: np.ndarray, into=None) -> torch.Tensor:
         raw = np.ascontiguousarray(arr).view(np.uint8).reshape(-1)
         nb = raw.size
         if nb > self.slot_bytes:  # rare: larger than a slot
-            return torch.from_numpy(np.ascontiguousarray(arr)).to(self.device)
+            host = torch.from_numpy(np.ascontiguousarray(arr))
+            return host.to(self.device) if into is None else into.copy_(host)
         i = self.next
         self.next = (i + 1) % len(self.slots)
         if self.events[i] is not None:
             self.events[i].synchronize()
         self.views[i][:nb] = raw
-        dev = torch.empty(nb, dtype=torch.uint8, device=self.device)
+        dev = torch.empty(nb, dtype=torch.uint8, device=self.device) if into is None else into
         dev.copy_(self.slots[i][:nb], non_blocking=True)
         ev = torch.cuda.Event()
         ev.record(torch.cuda.current_stream(self.device))
@@ -74,13 +75,16 @@ class _PinnedRing:
 _rings = {}
 
 
-def upload(arr: np.ndarray, device, dtype=None, shape=None) -> torch.Tensor:
-    """Copy a host array to the device asynchronously (stream-ordered)."""
+def upload(arr: np.ndarray, device, dtype=None, shape=None, into=None) -> torch.Tensor:
+    """Copy a host array to the device asynchronously (stream-ordered); ``into``
+    (uint8, the array's bytes) receives it if given."""
     key = torch.device(device).index or 0
     ring = _rings.get(key)
     if ring is None:
         ring = _rings[key] = _PinnedRing(torch.device(device))
-    dev = ring.upload(arr)
+    dev = ring.upload(arr, into)
+    if into is not None:
+        return into
     tdt = dtype if dtype is not None else {np.dtype(np.int64): torch.int64, np.dtype(np.complex64): torch.complex64,
                                            np.dtype(np.complex128): torch.complex128}[np.dtype(arr.dtype)]
     out = dev.view(tdt)
@@ -89,10 +93,6 @@ def upload(arr: np.ndarray, device, dtype=None, shape=None) -> torch.Tensor:
 
 def _dbits(x: float) -> int:
     return int(np.array([x], dtype=np.float64).view(np.int64)[0])
-
-
-def _bitsd(v: int) -> float:
-    return float(np.array([v], dtype=np.int64).view(np.float64)[0])
 
 
 class ResidentState:
@@ -132,35 +132,64 @@ def enter(mps):
     mps._res = ResidentState(mps)
 
 
-def leave(mps):
-    """Synchronise, turn the capacity buffers into the tensor list, log statistics."""
+class ReadBack:
+    """Bond dimensions and gate records of several states in two device-to-host
+    copies (they synchronise the stream).  One copy per state and round costs
+    ~12 us each: 168 of them for 24 instances of six rounds, 2 ms of the 5 that
+    leaving took, and the records' fields are unpacked per batch, not per gate."""
+
+    _REAL = [_lib.D_CONDS, _lib.D_ENTROPY, _lib.D_EPSLOC]
+    _INT = [_lib.D_STATUS, _lib.D_K, _lib.D_CHIM]
+
+    def __init__(self, states):
+        dims = states[0].dims if len(states) == 1 else torch.cat([r.dims for r in states])
+        flat, at = dims.cpu().tolist(), 0
+        self.dims = {}
+        for r in states:
+            self.dims[id(r)] = flat[at:at + len(r.bufs) + 1]
+            at += len(r.bufs) + 1
+        descs = {id(d): d for r in states for d, _, _ in r.batches}
+        self.rows = {}
+        if descs:
+            ds = list(descs.values())
+            out = (ds[0] if len(ds) == 1 else torch.cat(ds)).cpu().numpy()
+            ints, at = out[:, self._INT].tolist(), 0
+            reals = np.ascontiguousarray(out[:, self._REAL]).view(np.float64).tolist()
+            for d in ds:
+                G = d.shape[0]
+                self.rows[id(d)] = list(zip(ints[at:at + G], reals[at:at + G]))
+                at += G
+
+
+def leave(mps, back=None):
+    """Synchronise (or use a ``ReadBack`` that holds this state), turn the capacity
+    buffers into the tensor list, log statistics."""
     res = mps._res
     mps._res = None
-    dims = res.dims.cpu().tolist()  # synchronises the stream
+    if back is None:
+        back = ReadBack([res])
+    dims = back.dims[id(res)]
     n = mps.num_qubits
     mps._tensors = [res.bufs[s][:dims[s] * 2 * dims[s + 1]].view(dims[s], 2, dims[s + 1]) for s in range(n)]
     mps._bond_dims = dims[1:-1]
     err = None
     ngates = sum(len(rows) for _, rows, _ in res.batches)
     elapsed = (time.perf_counter() - res.batches[0][2]) * 1000.0 / max(ngates, 1) if res.batches else 0.0
+    dtype = str(res.dtype)
+    limit = mps.dtype_policy.promote_if_cond_gt if res.dtype != torch.complex128 else math.inf
     for desc_dev, rows, _ in res.batches:
-        out = desc_dev.cpu().numpy()
+        recs = back.rows[id(desc_dev)]
         for g, bond in rows:
-            row = out[g]
-            st = int(row[_lib.D_STATUS])
-            k = int(row[_lib.D_K])
-            cs = _bitsd(int(row[_lib.D_CONDS]))
+            (st, k, chiM), (cs, entropy, eps_local) = recs[g]
             drv = "gb300_gram_heevd_resident"
-            if math.isfinite(cs) and cs > mps.dtype_policy.promote_if_cond_gt and res.dtype != torch.complex128:
+            if math.isfinite(cs) and cs > limit:
                 drv = "gb300_gram_heevd_unpromoted"
                 mps.unpromoted += 1
             if st != _lib.AGB_OK and err is None:
                 err = (st, bond)
-            mps._last_entropy[bond] = _bitsd(int(row[_lib.D_ENTROPY]))
-            mps._log_operation(bond=bond, k_star=k, chi_before=int(row[_lib.D_CHIM]), chi_after=k,
-                               eps_local=_bitsd(int(row[_lib.D_EPSLOC])),
-                               entropy=_bitsd(int(row[_lib.D_ENTROPY])), svd_driver=drv, dtype=str(res.dtype),
-                               ms_elapsed=elapsed, condS=cs)
+            mps._last_entropy[bond] = entropy
+            mps._log_operation(bond=bond, k_star=k, chi_before=chiM, chi_after=k, eps_local=eps_local,
+                               entropy=entropy, svd_driver=drv, dtype=dtype, ms_elapsed=elapsed, condS=cs)
     if err is not None:
         check(err[0], f"two-site update on bond {err[1]} (device-resident batch)")
 
@@ -206,56 +235,52 @@ def single_qubit_entries(entries):
 
 
 def build_two_site(entries):
-    """Descriptor rows (host, int64) for resident two-site gates; plans them."""
+    """Descriptor rows (host, int64) for resident two-site gates; plans them.
+    Also returns the host-side gate matrices [j, 4, 4] (None if there are none)
+    and their rows, whose AGB_D_U the caller fills in."""
     lib = _lib.load()
     m0 = entries[0][0]
     dt = m0._res.dtype
     code = dtype_code(dt)
     G = len(entries)
-    desc = np.zeros((G, _lib.D_NFIELDS), dtype=np.int64)
     device = m0.device
     host_U, host_rows, keep = [], [], []
     seeds = {}
+    fields = []
     for g, (m, i, U) in enumerate(entries):
         res = m._res
         if res.dtype != dt:
             raise ValueError("resident batch entries must share the dtype")
-        row = desc[g]
-        row[_lib.D_A] = row[_lib.D_ANEW] = res.bufs[i].data_ptr()
-        row[_lib.D_B] = row[_lib.D_BNEW] = res.bufs[i + 1].data_ptr()
+        u = 0
         if U.device == device:
             if U.dtype != dt or not U.is_contiguous():
                 U = U.to(dtype=dt).contiguous()  # a device-side copy, no synchronisation
             keep.append(U)
-            row[_lib.D_U] = U.data_ptr()
+            u = U.data_ptr()
         else:
-            host_U.append(U.detach().to("cpu", dt).reshape(4, 4))
+            if U.dtype != dt or U.device.type != "cpu":
+                U = U.detach().to("cpu", dt)
+            host_U.append(U.reshape(4, 4))
             host_rows.append(g)
-        row[_lib.D_CHIL] = res.capL[i]
-        row[_lib.D_CHIM] = res.capb[i]
-        row[_lib.D_CHIR] = res.capR[i + 1]
-        row[_lib.D_CAP] = m.chi_max_per_bond[i]
-        row[_lib.D_EPS] = _dbits(m.eps_bond)
         j = seeds.get(id(m), 0)
         seeds[id(m)] = j + 1
-        row[_lib.D_SEED] = ((m._seed * 1000003 + m._operation_counter + len(res.batches)) & 0x3FFFFFFFFFFFFFFF) + j
-        row[_lib.D_DIMS] = res.dims.data_ptr()
-        row[_lib.D_BOND] = i
-        row[_lib.D_NVEC] = 0  # guided count; a short cut is repaired on the device
+        a, b = res.bufs[i].data_ptr(), res.bufs[i + 1].data_ptr()
+        fields.append((a, a, b, b, u, res.capL[i], res.capb[i], res.capR[i + 1], m.chi_max_per_bond[i],
+                       _dbits(m.eps_bond),
+                       ((m._seed * 1000003 + m._operation_counter + len(res.batches)) & 0x3FFFFFFFFFFFFFFF) + j,
+                       res.dims.data_ptr(), i))
+    desc = np.zeros((G, _lib.D_NFIELDS), dtype=np.int64)  # AGB_D_NVEC = 0: guided count, repaired on the device
+    desc[:, _TWO_SITE_FIELDS] = fields
     wsz = _lib.SZ(0)
     check(lib.agb_two_site_plan(code, G, desc.ctypes.data_as(ctypes.c_void_p), ctypes.byref(wsz)), "two_site_plan")
-    Ud = None
-    if host_U:
-        Ud = upload(torch.stack(host_U).numpy(), device)
-        keep.append(Ud)
-        for j, g in enumerate(host_rows):
-            desc[g, _lib.D_U] = Ud.data_ptr() + j * 16 * Ud.element_size()
-    maxL = int(desc[:, _lib.D_CHIL].max())
-    maxM = int(desc[:, _lib.D_CHIM].max())
-    maxR = int(desc[:, _lib.D_CHIR].max())
-    maxell = int(desc[:, _lib.D_ELL].max())
-    maxk = int(desc[:, _lib.D_CAP].max())
-    return desc, wsz.value, (maxL, maxM, maxR, maxell, maxk), keep
+    maxL, maxM, maxR, maxell, maxk = desc[:, [_lib.D_CHIL, _lib.D_CHIM, _lib.D_CHIR, _lib.D_ELL,
+                                              _lib.D_CAP]].max(axis=0).tolist()
+    Uh = torch.stack(host_U).detach().numpy() if host_U else None
+    return desc, wsz.value, (maxL, maxM, maxR, maxell, maxk), keep, Uh, host_rows
+
+
+_TWO_SITE_FIELDS = [_lib.D_A, _lib.D_ANEW, _lib.D_B, _lib.D_BNEW, _lib.D_U, _lib.D_CHIL, _lib.D_CHIM, _lib.D_CHIR,
+                    _lib.D_CAP, _lib.D_EPS, _lib.D_SEED, _lib.D_DIMS, _lib.D_BOND]
 
 
 def launch_two_site(code, G, desc_dev, ws, wsz, dims, stream):
@@ -271,9 +296,18 @@ def two_site_entries(entries):
     """Resident two-site gates of any number of instances, no host synchronisation."""
     m0 = entries[0][0]
     device = m0.device
-    desc, wsz, dims, keep = build_two_site(entries)
+    desc, wsz, dims, keep, Uh, host_rows = build_two_site(entries)
     ws = ops.workspace(wsz, device, "two_site_resident")
-    desc_dev = upload(desc, device)
+    if Uh is None:
+        desc_dev = upload(desc, device)
+    else:
+        # records and host gate matrices in one copy: the matrices follow the records
+        nb = desc.nbytes
+        buf = torch.empty(nb + Uh.nbytes, dtype=torch.uint8, device=device)
+        desc[host_rows, _lib.D_U] = buf.data_ptr() + nb + np.arange(len(host_rows), dtype=np.int64) * (16 * Uh.itemsize)
+        upload(np.concatenate((desc.view(np.uint8).reshape(-1), Uh.view(np.uint8).reshape(-1))), device, into=buf)
+        keep.append(buf)
+        desc_dev = buf[:nb].view(torch.int64).view(desc.shape)
     launch_two_site(dtype_code(m0._res.dtype), len(entries), desc_dev, ws, wsz, dims, stream_ptr(device))
     t = time.perf_counter()
     rows = {}
