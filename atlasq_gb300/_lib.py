@@ -78,6 +78,7 @@ _SIGS = {
     "agb_heevd": (I, [I, I, I, I, P, P, P, P, SZ, U64, P]),
     "agb_qr_workspace": (SZ, [I, I, I]),
     "agb_qr": (I, [I, P, I, I, I, P, P, I, P, SZ, P]),
+    "agb_qr_pair": (I, [I, P, P, SZ, P]),
     "agb_qr_noalloc": (I, [I, P, I, I, I, P, P, I, P]),
     "agb_sample_site": (I, [I, P, I, I, I, U64, U64, P, P, P, P]),
     "agb_mpo_mix": (I, [I, P, P, P, I, I, I, I, P]),

@@ -310,20 +310,23 @@ class AdaptiveMPS:
         self.to_left_canonical()
 
     @torch.no_grad()
-    def _right_sweep(self, tensors, stop=0):
-        """mps_pytorch.py:123-152 on a list, sites n-1 .. stop+1."""
-        for i in range(len(tensors) - 1, stop, -1):
+    def _right_sweep(self, tensors, stop=0, start=None):
+        """mps_pytorch.py:123-152 on a list, sites start (n-1) .. stop+1."""
+        for i in range(len(tensors) - 1 if start is None else start, stop, -1):
             Tm = self._common(tensors[i])
-            l, p, r = Tm.shape
-            Q, R = ops.qr(Tm.reshape(l, p * r), transA=True, trans_out=True)
-            kk = Q.shape[0]
-            tensors[i] = Q.reshape(kk, p, r)
-            prev = self._common(tensors[i - 1])
-            pl, pp, pr = prev.shape
-            tensors[i - 1] = ops.cgemm(prev.reshape(pl * pp, pr), R).reshape(pl, pp, kk)
-            if i - 1 < len(self._bond_dims):
-                self._bond_dims[i - 1] = kk
+            Q, R = ops.qr(Tm.reshape(Tm.shape[0], -1), transA=True, trans_out=True)
+            self._absorb_right(tensors, i, Q, R)
         return tensors
+
+    def _absorb_right(self, tensors, i, Q, R):
+        _, p, r = tensors[i].shape
+        kk = Q.shape[0]
+        tensors[i] = Q.reshape(kk, p, r)
+        prev = self._common(tensors[i - 1])
+        pl, pp, pr = prev.shape
+        tensors[i - 1] = ops.cgemm(prev.reshape(pl * pp, pr), R).reshape(pl, pp, kk)
+        if i - 1 < len(self._bond_dims):
+            self._bond_dims[i - 1] = kk
 
     @torch.no_grad()
     def canonicalize_right_to_left(self):
@@ -336,15 +339,34 @@ class AdaptiveMPS:
         assert 0 <= center < self.num_qubits, "Center out of range"
         self._flush()
         T = self._tensors
-        for i in range(center):
-            A = self._common(T[i])
-            l, p, r = A.shape
-            Q, R = ops.qr(A.reshape(l * p, r))
+        n = self.num_qubits
+
+        def from_left(i, Q, R):
+            l, p, _ = T[i].shape
             T[i] = Q.reshape(l, p, Q.shape[1])
             B = self._common(T[i + 1])
             T[i + 1] = ops.cgemm(R, B.reshape(B.shape[0], -1)).reshape(Q.shape[1], 2, B.shape[2])
             self._bond_dims[i] = Q.shape[1]
-        self._right_sweep(T, stop=center)
+
+        # the sweeps from the two ends meet only at the centre: their factorisations
+        # run in pairs; the centre takes the left sweep's factor first
+        both = min(center, n - 1 - center)
+        last = None
+        for s in range(both):
+            i, j = s, n - 1 - s
+            A, B = self._common(T[i]), self._common(T[j])
+            (Q, R), (Q2, R2) = ops.qr_pair(A.reshape(-1, A.shape[2]), B.reshape(B.shape[0], -1))
+            from_left(i, Q, R)
+            if j == center + 1 and center > both:
+                last = (j, Q2, R2)
+            else:
+                self._absorb_right(T, j, Q2, R2)
+        for i in range(both, center):
+            A = self._common(T[i])
+            from_left(i, *ops.qr(A.reshape(-1, A.shape[2])))
+        if last is not None:
+            self._absorb_right(T, *last)
+        self._right_sweep(T, stop=center, start=n - 1 - both)
 
     def _normalize(self):
         """mps_pytorch.py:595-604."""

@@ -107,10 +107,7 @@ def heevd(H, ell=None, seed=0):
     return (evals, evecs) if batched else (evals[0], evecs[0])
 
 
-def qr(A, transA=False, trans_out=False):
-    """Thin Householder QR of op(A); returns (Q, R) (or (Q^T, R^T) with trans_out)."""
-    lib = _lib.load()
-    A = _c(A)
+def _qr_outputs(A, transA, trans_out):
     M, N = (A.shape[1], A.shape[0]) if transA else (A.shape[0], A.shape[1])
     kk = min(M, N)
     if trans_out:
@@ -119,6 +116,31 @@ def qr(A, transA=False, trans_out=False):
     else:
         Q = torch.empty(M, kk, dtype=A.dtype, device=A.device)
         R = torch.empty(kk, N, dtype=A.dtype, device=A.device)
+    return M, N, Q, R
+
+
+def qr_pair(A, B):
+    """(Q, R) of A, and (Q^T, R^T) of B^T (``qr(B, transA=True, trans_out=True)``), of
+    one dtype and device, in one launch where both take the same form of the
+    blocked kernel."""
+    lib = _lib.load()
+    A, B = _c(A), _c(B)
+    code = dtype_code(A.dtype)
+    M, N, Q, R = _qr_outputs(A, False, False)
+    M2, N2, Q2, R2 = _qr_outputs(B, True, True)
+    need = lib.agb_qr_workspace(code, M, N) + lib.agb_qr_workspace(code, M2, N2)
+    ws = workspace(need, A.device, "qr")
+    probs = (ctypes.c_int64 * 14)(A.data_ptr(), M, N, 0, Q.data_ptr(), R.data_ptr(), 0,
+                                  B.data_ptr(), M2, N2, 1, Q2.data_ptr(), R2.data_ptr(), 1)
+    check(lib.agb_qr_pair(code, probs, ptr(ws), ws.numel(), stream_ptr(A.device)), "qr_pair")
+    return (Q, R), (Q2, R2)
+
+
+def qr(A, transA=False, trans_out=False):
+    """Thin Householder QR of op(A); returns (Q, R) (or (Q^T, R^T) with trans_out)."""
+    lib = _lib.load()
+    A = _c(A)
+    M, N, Q, R = _qr_outputs(A, transA, trans_out)
     need = lib.agb_qr_workspace(dtype_code(A.dtype), M, N)
     ws = workspace(need, A.device, "qr")
     check(lib.agb_qr(dtype_code(A.dtype), ptr(A), M, N, int(transA), ptr(Q), ptr(R), int(trans_out),

@@ -196,6 +196,10 @@ int agb_heevd(int dtype, int batch, int n, int ell, void* H, void* evals, void* 
 size_t agb_qr_workspace(int dtype, int M, int N);
 int agb_qr(int dtype, const void* A, int M, int N, int transA, void* Q, void* R, int trans_out,
            void* ws, size_t ws_bytes, void* stream);
+/* Two such factorisations, in one launch where both take the blocked cluster kernel
+ * with the same cluster size.  probs (host): [2][7] = {A, M, N, transA, Q, R, trans_out};
+ * ws holds both workspaces. */
+int agb_qr_pair(int dtype, const int64_t* probs, void* ws, size_t ws_bytes, void* stream);
 
 /* Allocation-free variant of agb_qr (no counterpart in the reference).
  * For callers that cannot allocate device memory -- e.g. a host runtime that
