@@ -29,8 +29,12 @@
 // panel, on one SM at a time: the panel is a chain of QB columns (norm, reflector,
 // barrier, product, update), the update of QB columns by QB reflectors is bound by
 // that SM's FP32 pipe (2 QB^2 M complex multiply-adds).
-// 512 x 256 on 16 CTAs: 0.62 ms (0.99 before): panels 24 us, updates 7.5, the
-// thin Q 6 us a panel.
+// Inside a panel 15 warps issue ~15 instructions a row for product and update of
+// each column (1400 of its 2800 cycles; the reflector 1200): the reflector is read
+// once, into registers, and in complex64 up to 512 rows padded with zeros to the
+// registers' rows, so that no access is predicated.  512 x 256 on 16 CTAs: 0.57 ms
+// (0.65 with predicated reads, twice a column); updates 8 us, the thin Q 6 us a
+// panel.
 #include <cooperative_groups.h>
 
 #include "householder.cuh"
@@ -52,7 +56,8 @@ struct QrbLayout {
   size_t panels, vloc, vloc2, w, w2, t, vb, total;  // byte offsets (vloc2 == vloc: one buffer of V)
 };
 
-AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C) {
+// vrows: rows of the two reflector buffers
+AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C, int vrows) {
   QrbLayout L;
   L.QB = QB;
   L.C = C;
@@ -68,7 +73,7 @@ AGB_HD QrbLayout qrb_layout(int esz, int QB, int M, int N, int C) {
   L.w = o;      o += (size_t)QB * L.npo * QB * esz;
   L.w2 = o;     o += (size_t)QB * L.npo * QB * esz;
   L.t = o;      o += (size_t)QB * QB * esz;
-  L.vb = o;     o += (size_t)2 * M * esz;
+  L.vb = o;     o += (size_t)2 * vrows * esz;
   // a second V buffer where it fits: the thin Q's panels are then read ahead
   if (o + (size_t)QB * L.ld * esz <= kQrbSmemBudget) {
     L.vloc2 = o;
@@ -199,7 +204,7 @@ struct QrbProb {
   int M, N, transA, trans_out;
 };
 
-template <typename CX, int NK>
+template <typename CX, int NK, bool PAD>
 __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, QrbProb<CX> pr1, int C) {
   const QrbProb<CX> pr = (int)blockIdx.x < C ? pr0 : pr1;
   const CX* __restrict__ Ain = pr.A;
@@ -211,7 +216,8 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
   const int q = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int kk = M < N ? M : N;
-  const QrbLayout Lo = qrb_layout(sizeof(CX), QB, M, N, C);
+  const int vrows = PAD ? 32 * NK : M;
+  const QrbLayout Lo = qrb_layout(sizeof(CX), QB, M, N, C, vrows);
   const int ld = Lo.ld;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CX* pan = (CX*)(smem_raw + Lo.panels);  // own panels: local column s * QB + jj
@@ -220,11 +226,12 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
   CX* W = (CX*)(smem_raw + Lo.w);
   CX* W2 = (CX*)(smem_raw + Lo.w2);
   CX* Tl = (CX*)(smem_raw + Lo.t);
-  CX* vbuf = (CX*)(smem_raw + Lo.vb);  // [2][M] the current reflector, double-buffered
+  CX* vbuf = (CX*)(smem_raw + Lo.vb);  // [2][vrows] the current reflector, double-buffered
   __shared__ int ycols[kQrbMaxCols];
   __shared__ int ycount;
   __shared__ CX taus[QB];
   constexpr int TP = QB + 1;
+  constexpr bool HOLD = NK * sizeof(CX) <= 128;  // the reflector stays in registers between product and update
   __shared__ CX Ssh[QB * TP], Tsh[QB * TP];
   // own panels: p = q + s * C
   const int nown = (q < Lo.P) ? (Lo.P - q + C - 1) / C : 0;
@@ -277,7 +284,7 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
       };
       for (int jj = 0; jj < bw; ++jj) {
         const int c = pb + jj;
-        CX* vb = vbuf + (size_t)(jj & 1) * M;
+        CX* vb = vbuf + (size_t)(jj & 1) * vrows;
         if (wid == jj) {
           Rt p0 = 0, p1 = 0;
           CX am = czero<CX>();
@@ -301,7 +308,7 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
             const int r = lane + 32 * k;
             const CX u = cmul(x[k], sc);
             const CX v = r > c ? u : r == c ? mk<CX>(1, 0) : czero<CX>();
-            if (r < M) vb[r] = v;
+            if (PAD || r < M) vb[r] = v;
             x[k] = r > c ? u : r == c ? mk<CX>(beta, 0) : x[k];  // v below the diagonal
           }
           if (lane == 0) taus[jj] = t;
@@ -311,10 +318,12 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
         // the earlier ones (x = v_w below its diagonal) it is conj(S[w][jj])
         if (wid != jj && wid < pw) {
           CX a0 = czero<CX>(), a1 = czero<CX>();
+          CX v[HOLD ? NK : 1];
 #pragma unroll
           for (int k = 0; k < NK; ++k) {
             const int r = lane + 32 * k;
-            const CX vr = r < M ? vb[r] : czero<CX>();  // zero above row c
+            const CX vr = PAD || r < M ? vb[r] : czero<CX>();  // zero above row c and past M
+            if (HOLD) v[HOLD ? k : 0] = vr;
             if (k & 1) cfmac(a1, vr, x[k]);
             else cfmac(a0, vr, x[k]);
           }
@@ -324,7 +333,8 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
 #pragma unroll
             for (int k = 0; k < NK; ++k) {
               const int r = lane + 32 * k;
-              if (r < M) x[k] = csub(x[k], cmul(vb[r], tw));
+              if (HOLD) x[k] = csub(x[k], cmul(v[HOLD ? k : 0], tw));
+              else if (PAD || r < M) x[k] = csub(x[k], cmul(vb[r], tw));
             }
           } else if (lane == 0) {
             Ssh[wid * TP + jj] = cconj(acc);
@@ -457,12 +467,17 @@ using QrbKernel = void (*)(QrbProb<CX>, QrbProb<CX>, int);
 // The instance whose per-lane register column (NK rows per lane) covers M rows;
 // nullptr above 1024 rows (512 for complex128, whose columns would spill).
 template <typename CX>
-QrbKernel<CX> qrb_kernel_for(int M) {
-  if (M <= 128) return qr_blocked_kernel<CX, 4>;
-  if (M <= 256) return qr_blocked_kernel<CX, 8>;
-  if (M <= 512) return qr_blocked_kernel<CX, 16>;
+QrbKernel<CX> qrb_kernel_for(int M, bool pad) {
   if constexpr (sizeof(CX) == 8) {
-    if (M <= 1024) return qr_blocked_kernel<CX, 32>;
+    if (pad && M <= 128) return qr_blocked_kernel<CX, 4, true>;
+    if (pad && M <= 256) return qr_blocked_kernel<CX, 8, true>;
+    if (pad && M <= 512) return qr_blocked_kernel<CX, 16, true>;
+  }
+  if (M <= 128) return qr_blocked_kernel<CX, 4, false>;
+  if (M <= 256) return qr_blocked_kernel<CX, 8, false>;
+  if (M <= 512) return qr_blocked_kernel<CX, 16, false>;
+  if constexpr (sizeof(CX) == 8) {
+    if (M <= 1024) return qr_blocked_kernel<CX, 32, false>;
   }
   return nullptr;
 }
@@ -470,15 +485,15 @@ QrbKernel<CX> qrb_kernel_for(int M) {
 // Cluster size for the blocked kernel: the largest of 16, 8, 4, 2 CTAs not
 // above the panel count whose shared memory fits; 0 if none.
 template <typename CX>
-int qrb_cluster_size(int M, int N, size_t* smem_out) {
-  const QrbKernel<CX> kern = qrb_kernel_for<CX>(M);
+int qrb_cluster_size(int M, int N) {
+  const QrbKernel<CX> kern = qrb_kernel_for<CX>(M, true);
   if (!kern) return 0;
   constexpr int QB = QrbCfg<CX>::QB;
   const int P = (N + QB - 1) / QB;
   static int allow16 = -1;
   for (int C : {16, 8, 4, 2}) {
     if (C > P) continue;
-    const QrbLayout L = qrb_layout(sizeof(CX), QB, M, N, C);
+    const QrbLayout L = qrb_layout(sizeof(CX), QB, M, N, C, M);
     if (L.total > kQrbSmemBudget || L.npo * QB > kQrbMaxCols) continue;
     if (C == 16) {
       if (allow16 < 0) {
@@ -506,7 +521,6 @@ int qrb_cluster_size(int M, int N, size_t* smem_out) {
       }
       if (!allow16) continue;
     }
-    if (smem_out) *smem_out = L.total;
     return C;
   }
   return 0;
@@ -527,15 +541,13 @@ size_t qr_blocked_workspace(int esz, int M, int N) {
 template <typename CX>
 static int launch_qrb(QrbProb<CX>* probs, int count, void* ws, size_t ws_bytes, cudaStream_t s) {
   constexpr int QB = QrbCfg<CX>::QB;
-  size_t smem = 0, at = 0;
+  size_t at = 0;
   int C = 0, maxM = 0;
   for (int i = 0; i < count; ++i) {
     QrbProb<CX>& p = probs[i];
-    size_t sm = 0;
-    const int c = qrb_cluster_size<CX>(p.M, p.N, &sm);
+    const int c = qrb_cluster_size<CX>(p.M, p.N);
     if (c == 0 || (i > 0 && c != C)) return AGB_ERR_UNSUPPORTED;
     C = c;
-    smem = sm > smem ? sm : smem;
     maxM = p.M > maxM ? p.M : maxM;
     const int kk = p.M < p.N ? p.M : p.N, PF = (kk + QB - 1) / QB;
     p.Vg = (CX*)((char*)ws + at);
@@ -543,7 +555,19 @@ static int launch_qrb(QrbProb<CX>* probs, int count, void* ws, size_t ws_bytes, 
     at += qr_blocked_workspace(sizeof(CX), p.M, p.N);
   }
   if (ws_bytes < at) return AGB_ERR_WORKSPACE;
-  const QrbKernel<CX> kern = qrb_kernel_for<CX>(maxM);
+  auto shared = [&](bool padded) {
+    size_t most = 0;
+    for (int i = 0; i < count; ++i) {
+      const int vrows = padded ? (maxM <= 128 ? 128 : maxM <= 256 ? 256 : 512) : probs[i].M;
+      const size_t sm = qrb_layout(sizeof(CX), QB, probs[i].M, probs[i].N, C, vrows).total;
+      most = sm > most ? sm : most;
+    }
+    return most;
+  };
+  // padded where there is such an instance and its buffers fit
+  const bool pad = sizeof(CX) == 8 && maxM <= 512 && shared(true) <= kQrbSmemBudget;
+  const size_t smem = shared(pad);
+  const QrbKernel<CX> kern = qrb_kernel_for<CX>(maxM, pad);
   if (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return AGB_ERR_UNSUPPORTED;
@@ -598,8 +622,8 @@ static int qr_pair(const int64_t* probs, void* ws, size_t ws_bytes, cudaStream_t
 
 // Two factorisations in one launch where both take the blocked kernel with the
 // same cluster size, one after the other otherwise.  512 x 256, then its mirror image:
-// 1314 us one after the other, 657 us side by side (a chain of 40 sites at chi 256 to
-// its mixed form: 16.9 -> 9.8 ms).
+// 1146 us one after the other, 573 us side by side (a chain of 40 sites at chi 256 to
+// its mixed form: 16.9 -> 9.8 ms at 657 us each).
 extern "C" int agb_qr_pair(int dtype, const int64_t* probs, void* ws, size_t ws_bytes, void* stream) {
   if (dtype != AGB_C64 && dtype != AGB_C128) return AGB_ERR_ARG;
   if (!probs || !ws) return AGB_ERR_ARG;
