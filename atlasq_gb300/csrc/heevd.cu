@@ -584,31 +584,40 @@ __global__ void __launch_bounds__(TB) invit_async_kernel(const HeevdProb* __rest
 // Clusters of the leading nvec eigenvalues (consecutive gaps <= tol), once per
 // problem: P.M (the polish scratch, free until the polish) receives the count
 // and the (t0, t1) pairs.
+// One warp per problem: 32 gaps at a time, a lane whose gap ends a cluster finds its
+// start among the boundaries before it (one thread walking the eigenvalues took
+// 47 us at n = 1024, 13 at n = 200; now 3).
 template <typename R>
-__global__ void cluster_list_kernel(const HeevdProb* __restrict__ probs, int count) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) cluster_list_kernel(const HeevdProb* __restrict__ probs, int count) {
+  const int b = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (b >= count) return;
   const HeevdProb P = probs[b];
   int* clist = (int*)P.M;
   const int ell = P.ell, nv = P.nvec;
   if (nv < 2 || P.skip_vectors) {
-    clist[0] = 0;
+    if (lane == 0) clist[0] = 0;
     return;
   }
   const R* lam = (const R*)P.lam;
   const R tol = cluster_tol(lam, ell, P.ctol);
-  int found = 0, s = 0;
-  for (int t = 1; t <= nv; ++t) {
-    if (t == nv || (lam[t - 1] - lam[t]) > tol) {
-      if (t - s > 1) {
-        clist[1 + 2 * found] = s;
-        clist[2 + 2 * found] = t;
-        ++found;
-      }
-      s = t;
+  int found = 0, s = 0;  // clusters listed, start of the open one
+  for (int tb = 1; tb <= nv; tb += 32) {
+    const int t = tb + lane;
+    const bool end = t <= nv && (t == nv || (lam[t - 1] - lam[t]) > tol);
+    const unsigned ends = __ballot_sync(0xffffffffu, end);
+    const unsigned before = ends & ((1u << lane) - 1u);
+    const int start = before ? tb + 31 - __clz(before) : s;
+    const bool listed = end && t - start > 1;
+    const unsigned lists = __ballot_sync(0xffffffffu, listed);
+    if (listed) {
+      const int at = found + __popc(lists & ((1u << lane) - 1u));
+      clist[1 + 2 * at] = start;
+      clist[2 + 2 * at] = t;
     }
+    found += __popc(lists);
+    if (ends) s = tb + 31 - __clz(ends);
   }
-  clist[0] = found;
+  if (lane == 0) clist[0] = found;
 }
 
 template <typename R>
@@ -827,8 +836,14 @@ __global__ void __launch_bounds__(256) orth_guard_kernel(HeevdProb* __restrict__
   const R l0 = lam[0];
   if (!(l0 > R(0))) return;
   const R floor_ = l0 * R(64) * (sizeof(R) == 4 ? R(5.96e-8) : R(1.11e-16));
+  // descending: the checked columns are [0, kl).  Counted by the block (a scan by
+  // every thread was nv dependent reads, 45 of 57 us at n = 1024)
   int kl = 0;
-  while (kl < nv && lam[kl] > floor_) ++kl;  // descending: the checked columns are [0, kl)
+  for (int k0 = 0; k0 < nv; k0 += blockDim.x) {
+    const int k = k0 + threadIdx.x, in = __syncthreads_count(k < nv && lam[k] > floor_);
+    kl += in;
+    if (in < (int)blockDim.x) break;
+  }
   const CX* M = (const CX*)P.M;
   float worst = 0.f, wworst = 0.f;
   for (int i = 1 + blockIdx.y; i < kl; i += gridDim.y) {
@@ -881,25 +896,38 @@ __global__ void __launch_bounds__(256) bt_pair_coef_kernel(const HeevdProb* __re
 //   s1 = tau_j (v_j^H z),  s2 = tau_{j-1} (v_{j-1}^H z - (v_{j-1}^H v_j) s1):
 // one pass forms the three dot products (the last one does not depend on z),
 // one pass applies both reflectors.
-template <typename CX, int NK, int WARPS>
+//
+// What bounds it: the issue of one to four warps a scheduler and the latency of
+// the four sums between the passes.  The rows are taken in groups whose loads
+// are in flight together, without a predicate (rows past n are zeros): with a
+// branch per 32 rows, which skips more of the zeros, every load waited alone.
+// One gate at chi 512 (m = n = 1024): 1571 -> 768 us, and 690 with one column a warp
+// on twice the SMs; 20 gates at chi 256: 533 -> 410 us.  complex128 is bound by the
+// FP64 pipe and keeps the finer skip.
+template <typename CX, int NK, int WARPS, int COLS>
 __global__ void __launch_bounds__(WARPS * 32) backtransform2_kernel(const HeevdProb* __restrict__ probs) {
   typedef typename cx_traits<CX>::R R;
   const HeevdProb P = probs[blockIdx.y];
   const int n = P.n, ell = P.ell, nv = P.nvec;
-  const int col0 = blockIdx.x * 2 * WARPS;
+  const int col0 = blockIdx.x * COLS * WARPS;
   if (col0 >= nv || n > NK * 32 || P.skip_vectors) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CX* vbuf = (CX*)smem_raw;  // [2 buffers][2 reflectors][NK * 32]
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int t0 = col0 + 2 * wid, t1 = t0 + 1;
-  const bool h0 = t0 < nv, h1 = t1 < nv;
+  constexpr int KG = sizeof(CX) == 8 ? 4 : 1;  // chunks of 32 rows per branch
+  constexpr bool TWO = COLS == 2;
+  for (int r = n + tid; r < NK * 32; r += WARPS * 32)  // rows past n: zero in every buffer
+#pragma unroll
+    for (int b = 0; b < 4; ++b) vbuf[b * NK * 32 + r] = czero<CX>();
+  const int t0 = col0 + COLS * wid, t1 = t0 + 1;
+  const bool h0 = t0 < nv, h1 = TWO && t1 < nv;
   const R* Y = (const R*)P.Y;
-  CX z0[NK], z1[NK];
+  CX z0[NK], z1[TWO ? NK : 1];
 #pragma unroll
   for (int k = 0; k < NK; ++k) {
     const int r = lane + 32 * k;
     z0[k] = (r < n && h0) ? mk<CX>(Y[(int64_t)r * ell + t0], 0) : czero<CX>();
-    z1[k] = (r < n && h1) ? mk<CX>(Y[(int64_t)r * ell + t1], 0) : czero<CX>();
+    if (TWO) z1[TWO ? k : 0] = (r < n && h1) ? mk<CX>(Y[(int64_t)r * ell + t1], 0) : czero<CX>();
   }
   const CX* H = (const CX*)P.H;
   const CX* tau = (const CX*)P.tau;
@@ -942,32 +970,44 @@ __global__ void __launch_bounds__(WARPS * 32) backtransform2_kernel(const HeevdP
     // v_{j-1}^H v_j, the same for every column: from bt_pair_coef_kernel
     const CX c = (j >= 1) ? pair_coef[(n - 2 - j) >> 1] : czero<CX>();
     CX d10 = czero<CX>(), d11 = czero<CX>(), d20 = czero<CX>(), d21 = czero<CX>();
-    // v_j and v_{j-1} are zero in rows < j: chunks of 32 rows below that are
+    // v_j and v_{j-1} are zero in rows < j and >= n: groups of 32 KG such rows are
     // skipped (a warp-uniform test, so the register arrays keep static indices)
 #pragma unroll
-    for (int k = 0; k < NK; ++k) {
-      const int r = lane + 32 * k;
-      if (32 * k + 31 >= j && r < n) {
-        const CX v1 = b1[r], v2 = b2[r];
-        cfmac(d10, v1, z0[k]);
-        cfmac(d11, v1, z1[k]);
-        cfmac(d20, v2, z0[k]);
-        cfmac(d21, v2, z1[k]);
+    for (int k0 = 0; k0 < NK; k0 += KG) {
+      if (32 * (k0 + KG) <= j || 32 * k0 >= n) continue;
+      CX v1[KG], v2[KG];
+#pragma unroll
+      for (int k = 0; k < KG; ++k) {
+        v1[k] = b1[lane + 32 * (k0 + k)];
+        v2[k] = b2[lane + 32 * (k0 + k)];
+      }
+#pragma unroll
+      for (int k = 0; k < KG; ++k) {
+        cfmac(d10, v1[k], z0[k0 + k]);
+        if (TWO) cfmac(d11, v1[k], z1[TWO ? k0 + k : 0]);
+        cfmac(d20, v2[k], z0[k0 + k]);
+        if (TWO) cfmac(d21, v2[k], z1[TWO ? k0 + k : 0]);
       }
     }
     d10 = warp_csum(d10);
-    d11 = warp_csum(d11);
+    if (TWO) d11 = warp_csum(d11);
     d20 = warp_csum(d20);
-    d21 = warp_csum(d21);
+    if (TWO) d21 = warp_csum(d21);
     const CX s10 = cmul(t1, d10), s11 = cmul(t1, d11);
     const CX s20 = cmul(t2, csub(d20, cmul(c, s10))), s21 = cmul(t2, csub(d21, cmul(c, s11)));
 #pragma unroll
-    for (int k = 0; k < NK; ++k) {
-      const int r = lane + 32 * k;
-      if (32 * k + 31 >= j && r < n) {
-        const CX v1 = b1[r], v2 = b2[r];
-        z0[k] = csub(z0[k], cadd(cmul(v1, s10), cmul(v2, s20)));
-        z1[k] = csub(z1[k], cadd(cmul(v1, s11), cmul(v2, s21)));
+    for (int k0 = 0; k0 < NK; k0 += KG) {
+      if (32 * (k0 + KG) <= j || 32 * k0 >= n) continue;
+      CX v1[KG], v2[KG];
+#pragma unroll
+      for (int k = 0; k < KG; ++k) {
+        v1[k] = b1[lane + 32 * (k0 + k)];
+        v2[k] = b2[lane + 32 * (k0 + k)];
+      }
+#pragma unroll
+      for (int k = 0; k < KG; ++k) {
+        z0[k0 + k] = csub(z0[k0 + k], cadd(cmul(v1[k], s10), cmul(v2[k], s20)));
+        if (TWO) z1[TWO ? k0 + k : 0] = csub(z1[TWO ? k0 + k : 0], cadd(cmul(v1[k], s11), cmul(v2[k], s21)));
       }
     }
   }
@@ -977,7 +1017,7 @@ __global__ void __launch_bounds__(WARPS * 32) backtransform2_kernel(const HeevdP
     const int r = lane + 32 * k;
     if (r < n) {
       if (h0) V[(int64_t)r * P.ldv + t0] = z0[k];
-      if (h1) V[(int64_t)r * P.ldv + t1] = z1[k];
+      if (h1) V[(int64_t)r * P.ldv + t1] = z1[TWO ? k : 0];
     }
   }
 }
@@ -990,7 +1030,11 @@ int launch_bt(const HeevdProb* probs, int count, int maxell, cudaStream_t s) {
   // SMs idled (each CTA stages every reflector pair once; the extra reads hit L2).
   constexpr int WARPS = 4;
   constexpr size_t smem = (size_t)4 * NK * 32 * sizeof(CX);
-  const cudaError_t oe = agb_smem_optin(backtransform2_kernel<CX, NK, WARPS>, smem);
+  // one column a warp where two leave SMs without a CTA (a single large gate)
+  const int pairs = (maxell + 2 * WARPS - 1) / (2 * WARPS);
+  const bool one = sizeof(CX) == 8 && pairs * count < 152;
+  auto kern = one ? backtransform2_kernel<CX, NK, WARPS, 1> : backtransform2_kernel<CX, NK, WARPS, 2>;
+  const cudaError_t oe = agb_smem_optin(kern, smem);
   if (oe != cudaSuccess) {
     agb_note_error(__FILE__, __LINE__, oe);
     return AGB_ERR_CUDA;
@@ -998,8 +1042,7 @@ int launch_bt(const HeevdProb* probs, int count, int maxell, cudaStream_t s) {
   const int npairs = NK * 32 / 2;  // pairs for the largest n this instance handles
   bt_pair_coef_kernel<CX><<<dim3((npairs + 7) / 8, count), 256, 0, s>>>(probs);
   AGB_CHECK_LAUNCH();
-  dim3 grid((maxell + 2 * WARPS - 1) / (2 * WARPS), count);
-  backtransform2_kernel<CX, NK, WARPS><<<grid, WARPS * 32, smem, s>>>(probs);
+  kern<<<dim3(one ? (maxell + WARPS - 1) / WARPS : pairs, count), WARPS * 32, smem, s>>>(probs);
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }
@@ -1084,7 +1127,7 @@ int launch_heevd_vectors(HeevdProb* probs, GemmProb* gp, int count, int maxn, in
       return AGB_ERR_CUDA;
     }
     const int maxcl = maxell / 2 > 0 ? maxell / 2 : 1;
-    cluster_list_kernel<R><<<(count + 127) / 128, 128, 0, s>>>(probs, count);
+    cluster_list_kernel<R><<<(count + 3) / 4, 128, 0, s>>>(probs, count);
     AGB_CHECK_LAUNCH();
     cluster_invit_kernel<R><<<dim3(maxcl, count), 256, sm, s>>>(probs, zcap);
     AGB_CHECK_LAUNCH();
@@ -1113,7 +1156,7 @@ int launch_heevd_vectors(HeevdProb* probs, GemmProb* gp, int count, int maxn, in
     AGB_CHECK_LAUNCH();
     if ((rc = launch_gemm_probs<CX>(gp, count, maxell, maxell, s, c, maxn))) return rc;
     if (step == 0) {
-      orth_guard_kernel<CX><<<dim3(count, 8), 256, 0, s>>>(probs);
+      orth_guard_kernel<CX><<<dim3(count, 32), 256, 0, s>>>(probs);
       AGB_CHECK_LAUNCH();
     }
     if ((rc = launch_gemm_probs<CX>(gp + count, count, maxn, maxell, s, c, maxell))) return rc;
