@@ -481,6 +481,67 @@ __global__ void __launch_bounds__(512) prerank_kernel(int64_t* __restrict__ desc
 }
 
 // ------------------------------------------------------------------ rank selection
+// Row splits of norms_kernel: at least 32 rows each, at most 32, and few enough for
+// S (ell + 1) doubles to fit the eigensolver's LU scratch (5 n ell reals).
+AGB_HD int norm_splits(int m, int n) {
+  int S = m / 32;
+  S = S < 32 ? S : 32;
+  S = S < n ? S : n;
+  return S > 1 ? S : 1;
+}
+
+// Sums of |.|^2 over the rows of one split: the nvec columns of A V (entries
+// 0 .. nvec-1 of the split's record in the LU scratch, which the vector phase is
+// done with) and all of X (entry ell).  Memory-bound: one CTA a gate, in the rank
+// kernel, read them at 70 GB/s (174 us at m = n = 1024, 75 us for 20 gates at 512);
+// now 22 and 18 us, the rank kernel 43 and 28.
+template <typename CX>
+__global__ void __launch_bounds__(256) norms_kernel(const int64_t* __restrict__ desc, const char* ws, int pass) {
+  typedef typename cx_traits<CX>::R R;
+  const int g = blockIdx.y;
+  const HeevdProb* hp = (const HeevdProb*)ws + g;
+  if (pass == 1 && !hp->redo) return;
+  const int64_t* D = desc + (int64_t)g * AGB_D_NFIELDS;
+  const int m = 2 * (int)D[AGB_D_CHIL], n = 2 * (int)D[AGB_D_CHIR], ell = (int)D[AGB_D_ELL];
+  const int S = norm_splits(m, n), q = blockIdx.x;
+  if (q >= S) return;
+  const char* slab = ws + D[AGB_D_WS];
+  const Slab Ls = slab_layout(m, n, ell, sizeof(CX));
+  const int r0 = (int)((int64_t)m * q / S), r1 = (int)((int64_t)m * (q + 1) / S);
+  double* out = (double*)hp->lu + (size_t)q * (ell + 1);
+  const int tid = threadIdx.x;
+  constexpr int nt = 256;
+  __shared__ double part[nt], red[32];
+  const CX* X = (const CX*)(slab + Ls.X);
+  SumAcc<R> xa;
+#pragma unroll 4
+  for (int64_t i = (int64_t)r0 * n + tid; i < (int64_t)r1 * n; i += nt) xa.add(cabs2(X[i]));
+  const double total = block_sum(xa.value(), red);
+  if (tid == 0) out[ell] = total;
+  if (D[AGB_D_MODE] == 1) return;
+  // cw consecutive columns a pass, one per thread; nt / cw groups share the rows
+  const CX* AV = (const CX*)(slab + Ls.AV);
+  const int nv = min(hp->nvec, ell);
+  const int cw = min(max(32, ((nv + 31) / 32) * 32), nt), G = nt / cw;
+  const int lt = tid % cw, grp = tid / cw;
+  for (int c0 = 0; c0 < nv; c0 += cw) {
+    const int t = c0 + lt;
+    SumAcc<R> ca;
+    if (grp < G && t < nv) {
+#pragma unroll 4
+      for (int r = r0 + grp; r < r1; r += G) ca.add(cabs2(AV[(int64_t)r * ell + t]));
+    }
+    part[tid] = ca.value();
+    __syncthreads();
+    if (grp == 0 && t < nv) {
+      double acc = 0;
+      for (int k = 0; k < G; ++k) acc += part[k * cw + lt];
+      out[t] = acc;
+    }
+    __syncthreads();
+  }
+}
+
 // One block per gate.  sigma_t^2 = ||AV[:, t]||^2, sorted descending; then the
 // reference rank rule with torch-CPU float32 semantics for complex64:
 //   E = cumsum(S*S) accumulated in double, each partial rounded to float32;
@@ -502,49 +563,34 @@ __global__ void __launch_bounds__(1024) rank_kernel(int64_t* __restrict__ desc, 
   const double eps = dbits(D[AGB_D_EPS]);
   char* slab = ws + D[AGB_D_WS];
   const Slab Ls = slab_layout(m, n, ell, sizeof(CX));
-  const CX* X = (const CX*)(slab + Ls.X);
-  const CX* AV = (const CX*)(slab + Ls.AV);
   double* sig2 = (double*)(slab + Ls.sig2);
   int* perm = (int*)(slab + Ls.perm);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* s_raw = (double*)smem_raw;  // [ell]
   double* s_sorted = s_raw + ell;     // [ell]
-  __shared__ double red[32];
   R* s_key = (R*)(s_sorted + 2 * (size_t)ell);  // [ell] sort keys (values are exact in R)
-  __shared__ double part[1024];
   const int tid = threadIdx.x, nt = blockDim.x;
-  // total = ||X||_F^2 to double accuracy
-  SumAcc<R> xa;
-  for (int64_t i = tid; i < (int64_t)m * n; i += nt) xa.add(cabs2(X[i]));
-  const double total_d = block_sum(xa.value(), red);
+  // total = ||X||_F^2 and the column norms of A V, to double accuracy, from the row
+  // splits norms_kernel summed
+  const HeevdProb* hp = (const HeevdProb*)ws;
+  const int S = norm_splits(m, n);
+  const double* parts = (const double*)hp[g].lu;
+  double total_d = 0;
+  for (int q = 0; q < S; ++q) total_d += parts[(size_t)q * (ell + 1) + ell];
   __shared__ int nonfinite;
   if (tid == 0) nonfinite = !isfinite(total_d);
   __syncthreads();
   const int mode0 = (int)D[AGB_D_MODE];
-  const HeevdProb* hp = (const HeevdProb*)ws;
   // values present: the nvec leading eigenvectors (all ell in the identity mode);
   // AV and V keep the row stride ell
   const int nv = (mode0 == 1) ? ell : min(hp[g].nvec, ell);
-  // column norms of AV: a pass covers cw consecutive columns (one per thread,
-  // coalesced along the row); G = nt / cw groups of threads split the rows and
-  // group 0 adds the groups' partials in a fixed order
   if (mode0 != 1) {
-    const int cw = min(max(32, ((nv + 31) / 32) * 32), nt), G = nt / cw;
-    const int lt = tid % cw, grp = tid / cw;
-    for (int c0 = 0; c0 < nv; c0 += cw) {
-      const int t = c0 + lt;
-      SumAcc<R> ca;
-      if (grp < G && t < nv)
-        for (int r = grp; r < m; r += G) ca.add(cabs2(AV[(int64_t)r * ell + t]));
-      part[tid] = ca.value();
-      __syncthreads();
-      if (grp == 0 && t < nv) {
-        double acc = 0;
-        for (int q = 0; q < G; ++q) acc += part[q * cw + lt];
-        s_raw[t] = acc;
-      }
-      __syncthreads();
+    for (int t = tid; t < nv; t += nt) {
+      double acc = 0;
+      for (int q = 0; q < S; ++q) acc += parts[(size_t)q * (ell + 1) + t];
+      s_raw[t] = acc;
     }
+    __syncthreads();
   }
   for (int t = tid; t < nv; t += nt) {
     double acc = s_raw[t];
@@ -773,6 +819,8 @@ int run_impl(int ng, int64_t* desc, int maxL, int maxM, int maxR, int maxell, ch
     if (rc) return rc;
     prof_mark(AGB_ST_RANK, s);
     const int pass = (flags & (AGB_RUN_REPAIR | AGB_RUN_REPAIR_LATER)) ? 0 : 2;
+    norms_kernel<CX><<<dim3(norm_splits(maxm, maxn), ng), 256, 0, s>>>(desc, ws, pass);
+    AGB_CHECK_LAUNCH();
     rank_kernel<CX><<<ng, 1024, 4 * (size_t)maxell * sizeof(double), s>>>(desc, ng, ws, pass, guard);
     AGB_CHECK_LAUNCH();
     if (!(flags & AGB_RUN_REPAIR)) {
@@ -791,6 +839,8 @@ int run_impl(int ng, int64_t* desc, int maxL, int maxM, int maxR, int maxell, ch
   rc = launch_gemm_probs<CX>(gp + 3 * ng, ng, maxm, maxell, s, &ctx, maxn);
   if (rc) return rc;
   prof_mark(AGB_ST_RANK, s);
+  norms_kernel<CX><<<dim3(norm_splits(maxm, maxn), ng), 256, 0, s>>>(desc, ws, 1);
+  AGB_CHECK_LAUNCH();
   rank_kernel<CX><<<ng, 1024, 4 * (size_t)maxell * sizeof(double), s>>>(desc, ng, ws, 1, guard);
   AGB_CHECK_LAUNCH();
   prof_mark(AGB_ST_GAP, s);
