@@ -68,22 +68,12 @@ AGB_DEV void tri_lu(const R* d, const R* e, int n, R lam, R piv, R* U0, R* U1, R
   R u0 = d[0] - lam, u1 = (n > 1) ? e[0] : R(0), u2 = 0;
   for (int i = 0; i < n - 1; ++i) {
     const R sub = e[i], nd = d[i + 1] - lam, ns = (i + 1 < n - 1) ? e[i + 1] : R(0);
-    R a0, a1, a2, m, pv;
-    if (fabs(u0) >= fabs(sub)) {
-      if (u0 == R(0)) u0 = piv;
-      m = sub / u0;
-      a0 = u0; a1 = u1; a2 = u2;
-      u0 = nd - m * u1;
-      u1 = ns - m * u2;
-      pv = 0;
-    } else {
-      m = u0 / sub;
-      a0 = sub; a1 = nd; a2 = ns;
-      const R nu0 = u1 - m * nd, nu1 = u2 - m * ns;
-      u0 = nu0;
-      u1 = nu1;
-      pv = 1;
-    }
+    const bool keep = fabs(u0) >= fabs(sub);  // selects: one division serves both cases
+    if (keep && u0 == R(0)) u0 = piv;
+    const R a0 = keep ? u0 : sub, a1 = keep ? u1 : nd, a2 = keep ? u2 : ns, pv = keep ? R(0) : R(1);
+    const R m = (keep ? sub : u0) / a0;
+    u0 = (keep ? nd : u1) - m * a1;
+    u1 = (keep ? ns : u2) - m * a2;
     u2 = 0;
     U0[i * L + t] = inv_pivot(a0, piv);
     U1[i * L + t] = a1;

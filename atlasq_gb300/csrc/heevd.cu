@@ -1,4 +1,6 @@
 // Batched Hermitian eigensolver kernels (see heevd.cuh for the stage list).
+#include <type_traits>
+
 #include "eigvec.cuh"
 #include "prof.cuh"
 
@@ -210,9 +212,42 @@ AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
   return cnt;
 }
 
+// The same count in double from the determinants p_i = (d_i - x) p_{i-1} -
+// e_{i-1}^2 p_{i-2} of the leading blocks (q_i = p_i / p_{i-1}; Givens): each p_i is
+// exact for a relative change of a few ulp in d_i - x and e_{i-1}^2, as each q_i is.
+// An FP64 division is a dependent chain of ~880 cycles here, the fused
+// multiply-add one of its instructions.  A zero p_i counts as the small negative
+// pivot above; the pair is rescaled by a power of two every eight steps (with
+// |d_i - x| and e^2 below 8 after the scaling of H, and no less than ulps apart
+// from zero, that is far from both ends of the range).
+AGB_DEV int sturm_count(const double* d, const double* e2, int n, double x) {
+  constexpr double tiny = 0x1p-200;
+  double p2 = 1.0, p1 = d[0] - x;
+  if (p1 == 0.0) p1 = -tiny;
+  int cnt = p1 < 0.0;
+  auto step = [&](int i) {
+    double p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
+    if (p == 0.0) p = -tiny * p1;
+    cnt += (int)((unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31);
+    p2 = p1;
+    p1 = p;
+  };
+  int i = 1;
+  for (; i + 8 <= n; i += 8) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) step(i + k);
+    const int h = max(__double2hiint(p1) & 0x7ff00000, __double2hiint(p2) & 0x7ff00000);
+    const double f = __hiloint2double(0x7fe00000 - h, 0);
+    p1 *= f;
+    p2 *= f;
+  }
+  for (; i < n; ++i) step(i);
+  return cnt;
+}
+
 // A warp per eigenvalue, WARPS of them per CTA: 8 for float; 2 for double, whose
-// divisions are bound by the FP64 pipe of the SM (10 problems of n = 96: 499 us,
-// 918 us on the 60 CTAs of 8 warps).
+// steps share the FP64 pipe of the SM (10 problems of n = 96: 215 us, 499 with a
+// division a step, 918 on a quarter of the CTAs).
 template <typename R, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __restrict__ probs) {
   const HeevdProb P = probs[blockIdx.y];
@@ -268,11 +303,14 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
 }
 
 // ------------------------------------------------------------------ stage 3
+// One warp per CTA for double, whose warps would share the SM's FP64 pipe (10 problems
+// of n = 96: 240 -> 224 us; the chain of the divisions remains).
+template <typename R> constexpr int kInvitTB = sizeof(R) == 8 ? 32 : 128;
 template <typename R>
-__global__ void __launch_bounds__(128) invit_kernel(const HeevdProb* __restrict__ probs) {
+__global__ void __launch_bounds__(kInvitTB<R>) invit_kernel(const HeevdProb* __restrict__ probs) {
   const HeevdProb P = probs[blockIdx.y];
   const int n = P.n, ell = P.ell, nv = P.nvec;
-  if (blockIdx.x * 128 >= nv) return;
+  if (blockIdx.x * kInvitTB<R> >= nv) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* d = (R*)smem_raw;
   R* e = d + n;
@@ -281,7 +319,7 @@ __global__ void __launch_bounds__(128) invit_kernel(const HeevdProb* __restrict_
     e[i] = (i < n - 1) ? ((const R*)P.e)[i] : R(0);
   }
   __syncthreads();
-  const int t = blockIdx.x * 128 + threadIdx.x;
+  const int t = blockIdx.x * kInvitTB<R> + threadIdx.x;
   if (t >= nv || P.skip_vectors) return;
   if (in_cluster((const R*)P.lam, nv, t, cluster_tol((const R*)P.lam, ell, P.ctol))) return;
   const R lam = ((const R*)P.lam)[t];
@@ -299,22 +337,14 @@ __global__ void __launch_bounds__(128) invit_kernel(const HeevdProb* __restrict_
   R u0 = d[0] - lam, u1 = (n > 1) ? e[0] : R(0), u2 = 0;
   for (int i = 0; i < n - 1; ++i) {
     const R sub = e[i], nd = d[i + 1] - lam, ns = (i + 1 < n - 1) ? e[i + 1] : R(0);
-    R a0, a1, a2, m, pv;
-    if (fabs(u0) >= fabs(sub)) {
-      if (u0 == R(0)) u0 = piv;
-      m = sub / u0;
-      a0 = u0; a1 = u1; a2 = u2;
-      u0 = nd - m * u1;
-      u1 = ns - m * u2;
-      pv = 0;
-    } else {
-      m = u0 / sub;
-      a0 = sub; a1 = nd; a2 = ns;
-      const R nu0 = u1 - m * nd, nu1 = u2 - m * ns;
-      u0 = nu0;
-      u1 = nu1;
-      pv = 1;
-    }
+    // selects, not a branch: one division serves both cases (the lanes of a warp
+    // exchange rows at different steps)
+    const bool keep = fabs(u0) >= fabs(sub);
+    if (keep && u0 == R(0)) u0 = piv;
+    const R a0 = keep ? u0 : sub, a1 = keep ? u1 : nd, a2 = keep ? u2 : ns, pv = keep ? R(0) : R(1);
+    const R m = (keep ? sub : u0) / a0;
+    u0 = (keep ? nd : u1) - m * a1;
+    u1 = (keep ? ns : u2) - m * a2;
     u2 = 0;
     U0[i * L + t] = inv_pivot(a0, piv);
     U1[i * L + t] = a1;
@@ -413,14 +443,21 @@ __global__ void __launch_bounds__(128) invit_kernel(const HeevdProb* __restrict_
 // Inverse iteration, complex64 path (float tridiagonal), for n <= 1024: the
 // same LU, start vectors and three solves as invit_kernel, with the iterate of
 // each thread's eigenvector kept in shared memory and the LU factors streamed
-// from L2 through a per-thread ring of cp.async copies issued AHEAD chunks of
-// CH steps before use.  The solves' recurrences are chains of multiply-adds
-// (reciprocal pivots), so with the operands already in shared memory a step
-// costs a few cycles instead of an L2 round trip every IB steps.  Each thread
-// reads only its own ring entries and its own iterate column: no block-level
-// synchronisation after the tridiagonal is staged.  TB threads per CTA.
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+// from L2 through a per-thread ring of cp.async copies.  The solves' recurrences
+// are chains of multiply-adds (reciprocal pivots), so with the operands already
+// in shared memory a step costs a few cycles instead of an L2 round trip.  Each
+// thread reads only its own ring entries and its own iterate column: no
+// block-level synchronisation after the tridiagonal is staged.
+//
+// What bounds it: instructions and dependent latency of one warp a scheduler (7
+// sweeps over n).  So what a step needs is kept small: the factors of four steps
+// are one 16-byte copy (l forward, 1/u0 and u1 backward), the row exchange is a bit
+// in shared memory, and u2, which only an exchange fills, comes from e.
+// One gate at chi 512 (n = 1024): 638 -> 275 us, 20 gates at chi 256 329 -> 143, 16 at
+// chi 100 134 -> 60 (per step five 4-byte copies, two divisions in either branch of
+// the exchange, and loads that waited for the stores before them).
+__device__ __forceinline__ void cp_async16(float4* dst, const float4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -429,146 +466,228 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-constexpr int kInvCH = 16, kInvNCH = 6;  // steps per chunk, chunks in the ring (5 in flight)
+constexpr int kInvTB = 32;               // threads per CTA: one warp, so that few vectors spread over the SMs
+constexpr int kInvQ = 4, kInvNCH = 6;  // groups of four steps per chunk, chunks in the ring (5 in flight)
 
-size_t invit_async_smem(int n, int tb) {
-  return ((size_t)2 * n + (size_t)n * tb + (size_t)3 * kInvNCH * kInvCH * tb) * sizeof(float);
+AGB_HD int inv_quads(int n) { return (n + 3) / 4; }
+size_t invit_async_smem(int n) {
+  const int tb = kInvTB;
+  // ring, iterates (whole groups), exchange bits, d, e (one entry more)
+  return ((size_t)2 * kInvNCH * kInvQ * 4 * tb + (size_t)inv_quads(n) * 4 * tb + (size_t)((n + 31) / 32) * tb +
+          2 * (size_t)n + 1) * sizeof(float);
 }
 
-template <int TB>
-__global__ void __launch_bounds__(TB) invit_async_kernel(const HeevdProb* __restrict__ probs) {
-  constexpr int CH = kInvCH, NCH = kInvNCH, RS = NCH * CH;  // ring steps per array
+__global__ void __launch_bounds__(32) invit_async_kernel(const HeevdProb* __restrict__ probs) {
+  constexpr int TB = kInvTB, CQ = kInvQ, NCH = kInvNCH, RQ = NCH * CQ;  // ring groups per array
   typedef float R;
   const HeevdProb P = probs[blockIdx.y];
-  const int n = P.n, ell = P.ell, nv = P.nvec;
+  const int n = P.n, ell = P.ell, nv = P.nvec, nq = inv_quads(n);
   if (blockIdx.x * TB >= nv || P.skip_vectors) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* d = (R*)smem_raw;            // [n]
-  R* e = d + n;                   // [n]
-  R* ys = e + n;                  // [n][TB] iterate column of each thread
-  R* ring = ys + (size_t)n * TB;  // [3][RS][TB] streamed factors
-  for (int i = threadIdx.x; i < n; i += TB) {
-    d[i] = ((const R*)P.d)[i];
-    e[i] = (i < n - 1) ? ((const R*)P.e)[i] : R(0);
-  }
-  __syncthreads();  // the last block-level barrier: threads may leave from here on
   const int tid = threadIdx.x, t = blockIdx.x * TB + tid;
+  float4* ring = (float4*)smem_raw + tid;              // [2][RQ][TB] streamed factors
+  R* ys = (R*)((float4*)smem_raw + 2 * RQ * TB) + tid;  // [4 nq][TB] iterate column of each thread
+  uint32_t* bits = (uint32_t*)(ys + (size_t)4 * nq * TB);  // [(n + 31) / 32][TB] row exchanges
+  R* d = (R*)(bits - tid + (size_t)((n + 31) / 32) * TB);  // [n]
+  R* e = d + n;                                         // [n + 1], e[n - 1] = e[n] = 0
+  R tnorm = 0;
+  for (int i = tid; i < n; i += TB) {
+    const R di = ((const R*)P.d)[i], ei = (i < n - 1) ? ((const R*)P.e)[i] : R(0);
+    d[i] = di;
+    e[i] = ei;
+    tnorm = fmax(tnorm, fabs(di) + fabs(ei) + (i ? fabs(((const R*)P.e)[i - 1]) : R(0)));
+  }
+  if (tid == 0) e[n] = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tnorm = fmax(tnorm, __shfl_xor_sync(0xffffffffu, tnorm, o));
+  __syncwarp();  // the last synchronisation: threads may leave from here on
   if (t >= nv) return;
   if (in_cluster((const R*)P.lam, nv, t, cluster_tol((const R*)P.lam, ell, P.ctol))) return;
   const R lam = ((const R*)P.lam)[t];
-  R tnorm = 0;
-  for (int i = 0; i < n; ++i) tnorm = fmax(tnorm, fabs(d[i]) + fabs(e[i]) + (i ? fabs(e[i - 1]) : R(0)));
   const R piv = rlim<R>::eps() * fmax(tnorm, rlim<R>::pivmin());
-  R* lu = (R*)P.lu;
+  // factors of steps 4 q .. 4 q + 3 of column t at [q * ell + t]; 12 ceil(n / 4) ell
+  // floats, within the scratch's 5 n ell (its rounding up to 256 bytes for n < 3)
   const int64_t L = ell;
-  R* U0 = lu;
-  R* U1 = lu + (int64_t)n * L;
-  R* U2 = lu + 2 * (int64_t)n * L;
-  R* Lm = lu + 3 * (int64_t)n * L;
-  R* Pv = lu + 4 * (int64_t)n * L;
-  tri_lu(d, e, n, lam, piv, U0, U1, U2, Lm, Pv, L, t);
-  __threadfence_block();  // the factor stores precede the copies that read them back
+  float4* Lm = (float4*)P.lu + t;
+  float4* U0 = Lm + (int64_t)nq * L;
+  float4* U1 = U0 + (int64_t)nq * L;
+  {  // LU with partial pivoting of T - lam I, as tri_lu
+    R u0 = d[0] - lam, u1 = (n > 1) ? e[0] : R(0);
+    uint32_t word = 0;
+    for (int q = 0; q < nq; ++q) {
+      R l4[4], a4[4], b4[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = 4 * q + k;
+        l4[k] = a4[k] = b4[k] = 0;
+        if (i < n - 1) {
+          const R sub = e[i], nd = d[i + 1] - lam, ns = e[i + 1];
+          // selects, not a branch: the lanes of a warp exchange rows at different
+          // steps, and one division then serves both cases
+          const bool keep = fabs(u0) >= fabs(sub);
+          if (keep && u0 == R(0)) u0 = piv;
+          const R den = keep ? u0 : sub, m = (keep ? sub : u0) / den;
+          const R r0 = keep ? nd : u1, r1 = keep ? u1 : nd;
+          const R s0 = keep ? ns : R(0), s1 = keep ? R(0) : ns;
+          u0 = r0 - m * r1;
+          u1 = s0 - m * s1;
+          word |= (keep ? 0u : 1u) << (i & 31);
+          l4[k] = m;
+          a4[k] = inv_pivot(den, piv);
+          b4[k] = r1;
+        } else if (i == n - 1) {
+          a4[k] = inv_pivot(u0, piv);
+        }
+      }
+      Lm[q * L] = make_float4(l4[0], l4[1], l4[2], l4[3]);
+      U0[q * L] = make_float4(a4[0], a4[1], a4[2], a4[3]);
+      U1[q * L] = make_float4(b4[0], b4[1], b4[2], b4[3]);
+      if ((q & 7) == 7 || q == nq - 1) {
+        bits[(q >> 3) * TB] = word;
+        word = 0;
+      }
+    }
+  }
+  __threadfence();  // the factor stores precede the copies that read them back
   // start vector: uniform in [-1, 1), four entries per Philox call (a Gaussian
   // start costs a Philox call plus Box-Muller per entry, half of this kernel's
   // instructions; inverse iteration only needs a start with a component along
   // the wanted vector)
   R nrm = 0;
   const uint64_t per = (uint64_t)((n + 3) / 4);
-  for (int i0 = 0; i0 < n; i0 += 4) {
-    const uint64_t idx = (uint64_t)t * per + (uint64_t)(i0 >> 2);
+  for (int q = 0; q < nq; ++q) {
+    const uint64_t idx = (uint64_t)t * per + (uint64_t)q;
     const philox_out o = philox4x32_10((uint32_t)idx, (uint32_t)(idx >> 32), 0x11u, 0x5EEDu, (uint32_t)P.seed,
                                        (uint32_t)(P.seed >> 32));
     const uint32_t w[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int i = i0 + k;
-      if (i < n) {
-        const R b = (R)(int32_t)w[k] * R(4.656612873077393e-10);  // 2^-31
-        ys[i * TB + tid] = b;
-        nrm += b * b;
-      }
+      const int i = 4 * q + k;
+      const R b = i < n ? (R)(int32_t)w[k] * R(4.656612873077393e-10) : R(0);  // 2^-31
+      ys[i * TB] = b;
+      if (i < n) nrm += b * b;
     }
   }
-  auto rg = [&](int a, int step) -> R* { return ring + ((size_t)a * RS + step % RS) * TB + tid; };
-  const int nf = n - 1;  // forward steps i = 0 .. n-2 (operands Pv[i], Lm[i])
+  // chunk c of the forward sweep (groups from the first) or the backward one (from the last)
   auto issue_f = [&](int c) {
-    for (int k = 0; k < CH; ++k) {
-      const int i = c * CH + k;
-      if (i < nf) {
-        cp_async4(rg(0, i), Pv + (int64_t)i * L + t);
-        cp_async4(rg(1, i), Lm + (int64_t)i * L + t);
-      }
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int q = c * CQ + k;
+      if (q < nq) cp_async16(ring + (q % RQ) * TB, Lm + q * L);
     }
     cp_async_commit();
   };
-  // backward steps j = 0 .. n-1 handle row i = n-1-j (operands U0, U1, U2 of row i)
   auto issue_b = [&](int c) {
-    for (int k = 0; k < CH; ++k) {
-      const int j = c * CH + k;
-      if (j < n) {
-        const int i = n - 1 - j;
-        cp_async4(rg(0, j), U0 + (int64_t)i * L + t);
-        cp_async4(rg(1, j), U1 + (int64_t)i * L + t);
-        cp_async4(rg(2, j), U2 + (int64_t)i * L + t);
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int j = c * CQ + k;
+      if (j < nq) {
+        cp_async16(ring + (j % RQ) * TB, U0 + (nq - 1 - j) * L);
+        cp_async16(ring + (RQ + j % RQ) * TB, U1 + (nq - 1 - j) * L);
       }
     }
     cp_async_commit();
   };
-  const int cf = (nf + CH - 1) / CH, cb = (n + CH - 1) / CH;
-  for (int it = 0; it < 3; ++it) {
-    const R s = R(1) / sqrt(fmax(nrm, rlim<R>::pivmin()));
-    // forward: apply P and L
-    for (int c = 0; c < NCH - 1; ++c) issue_f(c);
-    R bi = ys[tid] * s;
-    for (int c = 0; c < cf; ++c) {
-      issue_f(c + NCH - 1);  // an empty group past the end keeps the count uniform
-      cp_async_wait<NCH - 1>();  // chunk c has landed
-#pragma unroll 4
-      for (int k = 0; k < CH; ++k) {
-        const int i = c * CH + k;
-        if (i < nf) {
-          R bn = ys[(i + 1) * TB + tid] * s;
-          if (*rg(0, i) != R(0)) {
-            const R tmp = bi;
-            bi = bn;
-            bn = tmp;
-          }
-          ys[i * TB + tid] = bi;
-          bi = bn - *rg(1, i) * bi;
+  const int nc = (nq + CQ - 1) / CQ;
+  // The operands of a whole chunk are loaded before its chain of steps; only the
+  // chunk with the last rows tests each of them.
+  R x1, x2, bi;
+  auto forward = [&](int c, R s, auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    float4 l[CQ];
+    R y[4 * CQ];
+    uint32_t ex[CQ];
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int q = c * CQ + k;
+      if (FULL || q < nq) {
+        l[k] = ring[(q % RQ) * TB];
+        ex[k] = bits[(q >> 3) * TB] >> (4 * (q & 7));
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        y[4 * k + h] = FULL || 4 * q + h + 1 < n ? ys[(4 * q + h + 1) * TB] * s : R(0);
+    }
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int q = c * CQ + k;
+      const R lv[4] = {l[k].x, l[k].y, l[k].z, l[k].w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (FULL || 4 * q + h < n - 1) {
+          const bool sw = (ex[k] >> h) & 1u;
+          const R yh = y[4 * k + h], keep = sw ? yh : bi, bn = sw ? bi : yh;
+          ys[(4 * q + h) * TB] = keep;
+          bi = bn - lv[h] * keep;
+        }
+    }
+  };
+  auto backward = [&](int c, auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    float4 f0[CQ], f1[CQ];
+    R y[4 * CQ], p2[4 * CQ];
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int j = c * CQ + k, q = nq - 1 - j;
+      if (FULL || q >= 0) {
+        f0[k] = ring[(j % RQ) * TB];
+        f1[k] = ring[(RQ + j % RQ) * TB];
+        const uint32_t ex = bits[(q >> 3) * TB] >> (4 * (q & 7));
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          y[4 * k + h] = ys[(4 * q + h) * TB];
+          p2[4 * k + h] = (ex >> h) & 1u ? e[4 * q + h + 1] : R(0);
         }
       }
     }
-    ys[(n - 1) * TB + tid] = bi;
-    cp_async_wait<0>();  // no copy in flight into the ring before it is reused
-    // backward substitution with the reciprocal pivots
-    for (int c = 0; c < NCH - 1; ++c) issue_b(c);
-    R x1 = 0, x2 = 0;
-    nrm = 0;
-    for (int c = 0; c < cb; ++c) {
-      issue_b(c + NCH - 1);
-      cp_async_wait<NCH - 1>();
-#pragma unroll 4
-      for (int k = 0; k < CH; ++k) {
-        const int j = c * CH + k;
-        if (j < n) {
-          const int i = n - 1 - j;
-          const R x = (ys[i * TB + tid] - *rg(1, j) * x1 - *rg(2, j) * x2) * *rg(0, j);
-          ys[i * TB + tid] = x;
+#pragma unroll
+    for (int k = 0; k < CQ; ++k) {
+      const int q = nq - 1 - (c * CQ + k);
+      const R p0[4] = {f0[k].x, f0[k].y, f0[k].z, f0[k].w}, p1[4] = {f1[k].x, f1[k].y, f1[k].z, f1[k].w};
+#pragma unroll
+      for (int h = 3; h >= 0; --h)
+        if (FULL || (q >= 0 && 4 * q + h < n)) {
+          const R x = (y[4 * k + h] - p1[h] * x1 - p2[4 * k + h] * x2) * p0[h];
+          ys[(4 * q + h) * TB] = x;
           nrm += x * x;
           x2 = x1;
           x1 = x;
         }
-      }
+    }
+  };
+  for (int it = 0; it < 3; ++it) {
+    const R s = R(1) / sqrt(fmax(nrm, rlim<R>::pivmin()));
+    // forward: apply P and L
+    for (int c = 0; c < NCH - 1; ++c) issue_f(c);
+    bi = ys[0] * s;
+    for (int c = 0; c < nc; ++c) {
+      issue_f(c + NCH - 1);  // an empty group past the end keeps the count uniform
+      cp_async_wait<NCH - 1>();  // chunk c has landed
+      if (4 * CQ * (c + 1) < n) forward(c, s, std::true_type{});
+      else forward(c, s, std::false_type{});
+    }
+    ys[(n - 1) * TB] = bi;
+    cp_async_wait<0>();  // no copy in flight into the ring before it is reused
+    // backward substitution with the reciprocal pivots
+    for (int c = 0; c < NCH - 1; ++c) issue_b(c);
+    x1 = x2 = 0;
+    nrm = 0;
+    for (int c = 0; c < nc; ++c) {
+      issue_b(c + NCH - 1);
+      cp_async_wait<NCH - 1>();
+      if (4 * (nq - c * CQ) <= n && (c + 1) * CQ <= nq) backward(c, std::true_type{});
+      else backward(c, std::false_type{});
     }
     cp_async_wait<0>();
     if (!(nrm < R(1e300)) || !(nrm > R(0))) {  // overflow / breakdown: restart from a unit vector
-      for (int i = 0; i < n; ++i) ys[i * TB + tid] = (i == (t % n)) ? R(1) : R(0);
+      for (int i = 0; i < n; ++i) ys[i * TB] = (i == (t % n)) ? R(1) : R(0);
       nrm = 1;
     }
   }
   const R sc = R(1) / sqrt(fmax(nrm, rlim<R>::pivmin()));
-  R* Y = (R*)P.Y;
-  for (int i = 0; i < n; ++i) Y[(int64_t)i * L + t] = ys[i * TB + tid] * sc;
+  R* Y = (R*)P.Y + t;
+#pragma unroll 8
+  for (int i = 0; i < n; ++i) Y[(int64_t)i * L] = ys[i * TB] * sc;
 }
 
 // ------------------------------------------------------------------ stage 4
@@ -1096,20 +1215,16 @@ int launch_heevd_vectors(HeevdProb* probs, GemmProb* gp, int count, int maxn, in
   prof_mark(AGB_ST_INVIT, s);
   if (sizeof(R) == 4 && maxn <= 1024) {
     // complex64: iterate in shared memory, factors streamed by cp.async
-    const int tb = maxn <= 512 ? 64 : 32;
-    const size_t sm = invit_async_smem(maxn, tb);
-    const cudaError_t oe = tb == 64 ? agb_smem_optin(invit_async_kernel<64>, sm)
-                                    : agb_smem_optin(invit_async_kernel<32>, sm);
+    const size_t sm = invit_async_smem(maxn);
+    const cudaError_t oe = agb_smem_optin(invit_async_kernel, sm);
     if (oe != cudaSuccess) {
       agb_note_error(__FILE__, __LINE__, oe);
       return AGB_ERR_CUDA;
     }
-    if (tb == 64)
-      invit_async_kernel<64><<<dim3((maxell + 63) / 64, count), 64, sm, s>>>(probs);
-    else
-      invit_async_kernel<32><<<dim3((maxell + 31) / 32, count), 32, sm, s>>>(probs);
+    invit_async_kernel<<<dim3((maxell + kInvTB - 1) / kInvTB, count), kInvTB, sm, s>>>(probs);
   } else {
-    invit_kernel<R><<<dim3((maxell + 127) / 128, count), 128, sm_r, s>>>(probs);
+    constexpr int TB = kInvitTB<R>;
+    invit_kernel<R><<<dim3((maxell + TB - 1) / TB, count), TB, sm_r, s>>>(probs);
   }
   AGB_CHECK_LAUNCH();
   prof_mark(AGB_ST_CLUSTER, s);

@@ -1,5 +1,6 @@
-"""The back-transformation with one and with two columns per warp, and the split
-column norms of the rank selection.
+"""The back-transformation with one and with two columns per warp, bisection and
+inverse iteration at their chunk edges, and the split column norms of the rank
+selection.
 
 The two column counts do the same arithmetic per column, so a matrix alone (few
 columns: one per warp) and among copies (two per warp), reduced by the same number
@@ -45,6 +46,28 @@ def test_columns_per_warp(n, C, many):
                 assert lib.agb_set_tridiag_cluster(_lib.AGB_C64, n, count, 0, 512) == 0
     assert torch.equal(w1[0], w2[0])
     assert torch.equal(v1[0], v2[0])
+
+
+@pytest.mark.parametrize("dt,batch", [(torch.complex64, 2), (torch.complex128, 2)])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 15, 16, 17, 18, 20, 32, 33, 47, 64, 65, 100])
+def test_eigenpairs_against_64_bits(n, batch, dt):
+    """Chunks of 16 steps of the inverse iteration, and groups of eight steps of
+    the complex128 count.  Eigenvalues as backward stability gives them,
+    (2 n + 24) u ||H||; vectors orthonormal to n u after the polish and residuals of
+    the reduction's (8 n + 64) u ||H||."""
+    g = torch.Generator().manual_seed(n)
+    X = torch.randn(batch, n + 2, n, generator=g, dtype=torch.complex128)
+    H = (X.mH @ X).to(dt)
+    w, v = (t.cpu().to(torch.complex128) for t in ops.heevd(H.to(DEV)))
+    u = 2.0 ** -24 if dt == torch.complex64 else 2.0 ** -53
+    for b in range(batch):
+        A = H[b].to(torch.complex128)
+        ref = torch.linalg.eigvalsh(A).flip(0)
+        top = float(ref.abs().max())
+        assert float((w[b].real - ref).abs().max()) <= (2 * n + 24) * u * top
+        eye = torch.eye(n, dtype=torch.complex128)
+        assert float((v[b].mH @ v[b] - eye).abs().max()) <= (2 * n + 24) * u
+        assert float(torch.linalg.vector_norm(A @ v[b] - v[b] * w[b], dim=0).max()) <= (8 * n + 64) * u * top
 
 
 @pytest.mark.parametrize("dt", [torch.complex64, torch.complex128])
