@@ -190,54 +190,45 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(const HeevdProb* __restri
 }
 
 // ------------------------------------------------------------------ stage 2
-// Number of eigenvalues of T below x (Sturm sequence of the LDL^T pivots).
-// A pivot smaller than pm in magnitude is replaced by -pm BEFORE it is
-// counted, so the count and the recurrence see the same sign (LAPACK dlaebz's
-// order).  Replacing it only at the next step, after counting it as
-// non-negative, loses one eigenvalue whenever a pivot cancels to exactly 0:
-// in float32 that happened at x midway between two leading eigenvalues 1.6e-5
-// apart, bisection then returned a value between them and inverse iteration
-// produced two overlapping eigenvectors.
+// Number of eigenvalues of T below x: sign changes of the determinants p_i = (d_i - x)
+// p_{i-1} - e_{i-1}^2 p_{i-2} of the leading blocks (Givens).  Each p_i is exact for
+// a relative change of a few ulp in d_i - x and e_{i-1}^2, like the pivots q_i = p_i /
+// p_{i-1} of the LDL^T form, whose division is most of its chain (FP64 ~880 cycles
+// a step, float ~50).  A zero p_i counts as a small negative pivot, so the count and
+// the recurrence see the same sign.  The pair is rescaled by a power of two every U
+// steps (8 in double, 4 in float): |d_i - x| and e^2 are below 8 after the scaling of
+// H, and factors below the range's U-th root only occur for |x| far below the
+// tolerance.
+AGB_DEV unsigned sign_bits(float a, float b) { return (unsigned)(__float_as_int(a) ^ __float_as_int(b)) >> 31; }
+AGB_DEV unsigned sign_bits(double a, double b) { return (unsigned)(__double2hiint(a) ^ __double2hiint(b)) >> 31; }
+// 2^-exponent of the larger of a and b
+AGB_DEV float pair_scale(float a, float b) {
+  const int h = max(__float_as_int(a) & 0x7f800000, __float_as_int(b) & 0x7f800000);
+  return __int_as_float(0x7f000000 - h);
+}
+AGB_DEV double pair_scale(double a, double b) {
+  const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
+  return __hiloint2double(0x7fe00000 - h, 0);
+}
 template <typename R>
 AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
-  const R pm = rlim<R>::pivmin();
-  R q = d[0] - x;
-  if (fabs(q) < pm) q = -pm;
-  int cnt = q < R(0);
-  for (int i = 1; i < n; ++i) {
-    q = d[i] - x - e2[i - 1] / q;
-    if (fabs(q) < pm) q = -pm;
-    cnt += q < R(0);
-  }
-  return cnt;
-}
-
-// The same count in double from the determinants p_i = (d_i - x) p_{i-1} -
-// e_{i-1}^2 p_{i-2} of the leading blocks (q_i = p_i / p_{i-1}; Givens): each p_i is
-// exact for a relative change of a few ulp in d_i - x and e_{i-1}^2, as each q_i is.
-// An FP64 division is a dependent chain of ~880 cycles here, the fused
-// multiply-add one of its instructions.  A zero p_i counts as the small negative
-// pivot above; the pair is rescaled by a power of two every eight steps (with
-// |d_i - x| and e^2 below 8 after the scaling of H, and no less than ulps apart
-// from zero, that is far from both ends of the range).
-AGB_DEV int sturm_count(const double* d, const double* e2, int n, double x) {
-  constexpr double tiny = 0x1p-200;
-  double p2 = 1.0, p1 = d[0] - x;
-  if (p1 == 0.0) p1 = -tiny;
-  int cnt = p1 < 0.0;
+  constexpr int U = sizeof(R) == 8 ? 8 : 4;
+  constexpr R tiny = sizeof(R) == 8 ? R(0x1p-200) : R(0x1p-60f);
+  R p2 = 1, p1 = d[0] - x;
+  if (p1 == R(0)) p1 = -tiny;
+  int cnt = p1 < R(0);
   auto step = [&](int i) {
-    double p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
-    if (p == 0.0) p = -tiny * p1;
-    cnt += (int)((unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31);
+    R p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
+    if (p == R(0)) p = -tiny * p1;
+    cnt += (int)sign_bits(p, p1);
     p2 = p1;
     p1 = p;
   };
   int i = 1;
-  for (; i + 8 <= n; i += 8) {
+  for (; i + U <= n; i += U) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) step(i + k);
-    const int h = max(__double2hiint(p1) & 0x7ff00000, __double2hiint(p2) & 0x7ff00000);
-    const double f = __hiloint2double(0x7fe00000 - h, 0);
+    for (int k = 0; k < U; ++k) step(i + k);
+    const R f = pair_scale(p1, p2);
     p1 *= f;
     p2 *= f;
   }
@@ -247,7 +238,8 @@ AGB_DEV int sturm_count(const double* d, const double* e2, int n, double x) {
 
 // A warp per eigenvalue, WARPS of them per CTA: 8 for float; 2 for double, whose
 // steps share the FP64 pipe of the SM (10 problems of n = 96: 215 us, 499 with a
-// division a step, 918 on a quarter of the CTAs).
+// division a step, 918 on a quarter of the CTAs).  float, with and without the
+// division: one problem of n = 1024 259 and 96 us, 20 of n = 512 199 and 105.
 template <typename R, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __restrict__ probs) {
   const HeevdProb P = probs[blockIdx.y];
