@@ -1,23 +1,13 @@
-// SIMT batched complex GEMM for sm_103a, 256 threads, K-step 16.  complex64:
-// 64 x 64 or 32 x 32 output tiles (launch_simt), for small and ragged shapes.
-// complex128: 16 x 16 tiles, one output per thread: the FP64 pipe does 2 lanes per clock and SM whatever the tile, so what counts is
-// how many SMs a product spreads over and how little of a ragged tile is
-// padding (a 10-gate layer at chi 48: 189 us over its 19 launches, 2043 us with
+// SIMT batched complex GEMM for sm_103a, 256 threads.  complex64: 64 x 64 or
+// 32 x 32 output tiles (launch_simt), for small and ragged shapes.  complex128:
+// 16 x 16 tiles, one output per thread: the FP64 pipe does 2 lanes per clock and SM
+// whatever the tile, so what counts is how many SMs a product spreads over and how
+// little of a ragged tile is padding (a 10-gate layer at chi 48: 189 us over its 19 launches, 2043 us with
 // 64 x 64 tiles, 40 CTAs a launch and a third of their area padding).
 #include "gemm.cuh"
 #include "gemm_tc.cuh"
 
 namespace {
-
-template <typename CX>
-AGB_DEV CX load_op(const CX* P, int64_t ld, int op, int row, int col, int rows, int cols) {
-  // element (row, col) of op(P), where op(P) is rows x cols
-  if (row >= rows || col >= cols) return czero<CX>();
-  if (op == 0) return P[(int64_t)row * ld + col];
-  if (op == 3) return cconj(P[(int64_t)row * ld + col]);
-  CX v = P[(int64_t)col * ld + row];
-  return op == 2 ? cconj(v) : v;
-}
 
 struct StridedBatch {
   GemmProb base;
@@ -56,35 +46,46 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
 #pragma unroll
     for (int j = 0; j < T; ++j) acc[i][j] = czero<CX>();
 
-  // A tile: BM x BK of op(A); B tile: BK x BN of op(B).  The next K step is read
-  // into registers while the current one is multiplied, and the two
-  // shared-memory buffers leave one barrier per step.
+  // A tile: BM x BK of op(A); B tile: BK x BN of op(B).  The next two K steps are
+  // read into registers while one is multiplied (a step is shorter than the
+  // latency of L2), and the two shared-memory buffers leave one barrier per step.
   constexpr int NE = BM * BK / 256;
-  const bool an = p.opA == 0 || p.opA == 3, bn = p.opB == 0 || p.opB == 3;
-  CX va[NE], vb[NE];
-  auto fetch = [&](int k0) {
+  const bool an = p.opA == 0 || p.opA == 3, bn = p.opB == 0 || p.opB == 3;  // K along a row / down a column
+  const bool conja = p.opA >= 2, conjb = p.opB >= 2;
+  const CX *pa[NE], *pb[NE];  // this thread's elements of the next step to read
+  int ka[NE], kb[NE];         // their K index, past K for rows and columns outside
+  const int64_t stepa = an ? BK : BK * p.lda, stepb = bn ? BK * p.ldb : BK;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    const int idx = tid + e * 256;
+    const int r = an ? idx / BK : idx % BM, c = an ? idx % BK : idx / BM;
+    pa[e] = A + (an ? (int64_t)(m0 + r) * p.lda + c : (int64_t)c * p.lda + m0 + r);
+    ka[e] = m0 + r < p.M ? c : p.K;
+    const int kr = bn ? idx / BN : idx % BK, nc = bn ? idx % BN : idx / BK;
+    pb[e] = B + (bn ? (int64_t)kr * p.ldb + n0 + nc : (int64_t)(n0 + nc) * p.ldb + kr);
+    kb[e] = n0 + nc < p.N ? kr : p.K;
+  }
+  CX va[2][NE], vb[2][NE];
+  auto fetch = [&](int k0, CX (&xa)[NE], CX (&xb)[NE]) {
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
-      const int idx = tid + e * 256;
-      const int r = an ? idx / BK : idx % BM, c = an ? idx % BK : idx / BM;
-      va[e] = load_op(A, p.lda, p.opA, m0 + r, k0 + c, p.M, p.K);
-      const int kr = bn ? idx / BN : idx % BK, nc = bn ? idx % BN : idx / BK;
-      vb[e] = load_op(B, p.ldb, p.opB, k0 + kr, n0 + nc, p.K, p.N);
+      xa[e] = k0 + ka[e] < p.K ? *pa[e] : czero<CX>();
+      xb[e] = k0 + kb[e] < p.K ? *pb[e] : czero<CX>();
+      pa[e] += stepa;
+      pb[e] += stepb;
     }
   };
-  fetch(0);
-  int buf = 0;
-  for (int k0 = 0; k0 < p.K; k0 += BK, buf ^= 1) {
+  auto step = [&](int k0, int buf, CX (&xa)[NE], CX (&xb)[NE]) {
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
       const int idx = tid + e * 256;
       const int r = an ? idx / BK : idx % BM, c = an ? idx % BK : idx / BM;
-      As[buf][c][r] = va[e];
+      As[buf][c][r] = conja ? cconj(xa[e]) : xa[e];
       const int kr = bn ? idx / BN : idx % BK, nc = bn ? idx % BN : idx / BK;
-      Bs[buf][kr][nc] = vb[e];
+      Bs[buf][kr][nc] = conjb ? cconj(xb[e]) : xb[e];
     }
     __syncthreads();
-    if (k0 + BK < p.K) fetch(k0 + BK);
+    if (k0 + 2 * BK < p.K) fetch(k0 + 2 * BK, xa, xb);
     const int kn = min(BK, p.K - k0);
     if (T == 1 && kn < BK) {  // no padding products on the FP64 pipe
       for (int k = 0; k < kn; ++k) cfma(acc[0][0], As[buf][k][ty], Bs[buf][k][tx]);
@@ -102,6 +103,12 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
           for (int j = 0; j < T; ++j) cfma(acc[i][j], a[i], b[j]);
       }
     }
+  };
+  fetch(0, va[0], vb[0]);
+  if (BK < p.K) fetch(BK, va[1], vb[1]);
+  for (int k0 = 0; k0 < p.K; k0 += 2 * BK) {
+    step(k0, 0, va[0], vb[0]);
+    if (k0 + BK < p.K) step(k0 + BK, 1, va[1], vb[1]);
   }
   const CX alpha = mk<CX>((R)p.alpha_re, (R)p.alpha_im);
   const CX beta = mk<CX>((R)p.beta_re, (R)p.beta_im);
@@ -126,10 +133,12 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
 
 }  // namespace
 
-// complex64: 64 x 64 tiles where they give every SM one, else 32 x 32 (a 256 x
-// 512 x 256 product: 32 CTAs of 64 x 64 take 40 us, 128 of 32 x 32 23; five
-// 200 x 400 x 200: 33 against 31; but 16384 x 64 x 16: 6.9 against 8.2).  With one
-// tile size, K-step 8 and no read-ahead: 55, 44 and 7.2 us.
+// complex64: 64 x 64 tiles (K-step 16) where they give every SM one, else 32 x 32
+// (K-step 32).  32 x 32 tiles are bound by the latency of a step, so it is long, and
+// two are read ahead from addresses formed once: a 256 x 512 x 256 product takes
+// 12.4 us (16.1 with K-step 16; 23 reading one step ahead, 27 with a transposed
+// operand; 32 CTAs of 64 x 64 took 40), five 200 x 400 x 200 27 (30), 64^3 5.2
+// (7.3), 1024^3 on 64 x 64 tiles 221 (248).
 template <typename CX>
 static int launch_simt(const GemmProb* probs, const StridedBatch& sb, int count, int64_t M, int64_t N,
                        cudaStream_t s) {
@@ -143,7 +152,7 @@ static int launch_simt(const GemmProb* probs, const StridedBatch& sb, int count,
     gemm_simt_kernel<CX, 16, 16, 1><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
   } else {
     if (b == 64) gemm_simt_kernel<CX, 64, 16, 4><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
-    else gemm_simt_kernel<CX, 32, 16, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    else gemm_simt_kernel<CX, 32, 32, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
   }
   AGB_CHECK_LAUNCH();
   return AGB_OK;
