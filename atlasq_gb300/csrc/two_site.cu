@@ -181,8 +181,8 @@ __global__ void __launch_bounds__((TL / S) * (TL / S)) contract_gate_kernel(cons
   const ContractProb P = probs ? probs[blockIdx.z] : single;
   const int l0 = blockIdx.y * TL, j0 = blockIdx.x * TL;
   if (l0 >= P.chiL || j0 >= P.chiR) return;
-  __shared__ Pair As[KC][TL + 1];  // [r][l]: p' = 0, 1 side by side
-  __shared__ Pair Bs[KC][TL + 1];  // [r][j]: q' = 0, 1
+  __shared__ Pair As[2][KC][TL + 1];  // [r][l]: p' = 0, 1 side by side
+  __shared__ Pair Bs[2][KC][TL + 1];  // [r][j]: q' = 0, 1
   __shared__ CX Us[16];
   const int tid = threadIdx.x, tx = tid % W, ty = tid / W;
   const CX* A = (const CX*)P.A;
@@ -194,45 +194,56 @@ __global__ void __launch_bounds__((TL / S) * (TL / S)) contract_gate_kernel(cons
 #pragma unroll
     for (int b = 0; b < S; ++b) th[a][b][0][0] = th[a][b][0][1] = th[a][b][1][0] = th[a][b][1][1] = czero<CX>();
   const int chiM = P.chiM, chiR = P.chiR, chiL = P.chiL;
-  // the next chunk is read into registers while the current one is multiplied
+  // the next DEPTH chunks are read into registers while one is multiplied: two with
+  // one output block per thread, whose chunk is shorter than the latency of L2
+  constexpr int DEPTH = TL == 16 ? 2 : 1;
   constexpr int NE = 2 * TL * KC / NT;
-  CX va[NE], vb[NE];
-  auto fetch = [&](int r0) {
+  const CX *pa[NE], *pb[NE];
+  int ka[NE], kb[NE];  // index along the middle bond, past its end for rows outside
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    const int idx = tid + NT * e;
+    {  // A[l][p][r]: r fastest
+      const int r = idx % KC, pp = (idx / KC) & 1, gl = l0 + idx / (2 * KC);
+      pa[e] = A + ((int64_t)gl * 2 + pp) * chiM + r;
+      ka[e] = gl < chiL ? r : chiM;
+    }
+    {  // B[r][q][j]: j fastest
+      const int gj = j0 + idx % TL, qq = (idx / TL) & 1, r = idx / (2 * TL);
+      pb[e] = B + ((int64_t)r * 2 + qq) * chiR + gj;
+      kb[e] = gj < chiR ? r : chiM;
+    }
+  }
+  const int64_t stepb = (int64_t)KC * 2 * chiR;
+  CX va[DEPTH][NE], vb[DEPTH][NE];
+  auto fetch = [&](int r0, CX (&xa)[NE], CX (&xb)[NE]) {
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
-      const int idx = tid + NT * e;
-      {  // A[l][p][r]: r fastest
-        const int r = idx % KC, pp = (idx / KC) & 1, l = idx / (2 * KC);
-        const int gl = l0 + l, gr = r0 + r;
-        va[e] = (gl < chiL && gr < chiM) ? A[((int64_t)gl * 2 + pp) * chiM + gr] : czero<CX>();
-      }
-      {  // B[r][q][j]: j fastest
-        const int j = idx % TL, qq = (idx / TL) & 1, r = idx / (2 * TL);
-        const int gr = r0 + r, gj = j0 + j;
-        vb[e] = (gr < chiM && gj < chiR) ? B[((int64_t)gr * 2 + qq) * chiR + gj] : czero<CX>();
-      }
+      xa[e] = r0 + ka[e] < chiM ? *pa[e] : czero<CX>();
+      xb[e] = r0 + kb[e] < chiM ? *pb[e] : czero<CX>();
+      pa[e] += KC;
+      pb[e] += stepb;
     }
   };
-  fetch(0);
-  for (int r0 = 0; r0 < chiM; r0 += KC) {
+  auto step = [&](int r0, int buf, CX (&xa)[NE], CX (&xb)[NE]) {
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
       const int idx = tid + NT * e;
-      CX* as = &As[idx % KC][idx / (2 * KC)].a;
-      as[(idx / KC) & 1] = va[e];
-      CX* bs = &Bs[idx / (2 * TL)][idx % TL].a;
-      bs[(idx / TL) & 1] = vb[e];
+      CX* as = &As[buf][idx % KC][idx / (2 * KC)].a;
+      as[(idx / KC) & 1] = xa[e];
+      CX* bs = &Bs[buf][idx / (2 * TL)][idx % TL].a;
+      bs[(idx / TL) & 1] = xb[e];
     }
     __syncthreads();
-    if (r0 + KC < chiM) fetch(r0 + KC);
+    if (r0 + DEPTH * KC < chiM) fetch(r0 + DEPTH * KC, xa, xb);
     const int rn = sizeof(CX) == 16 ? min(KC, chiM - r0) : KC;  // no padding products on the FP64 pipe
 #pragma unroll (sizeof(CX) == 16 ? 1 : KC)
     for (int r = 0; r < rn; ++r) {
       Pair a[S], b[S];
 #pragma unroll
       for (int k = 0; k < S; ++k) {
-        a[k] = As[r][ty + W * k];
-        b[k] = Bs[r][tx + W * k];
+        a[k] = As[buf][r][ty + W * k];
+        b[k] = Bs[buf][r][tx + W * k];
       }
 #pragma unroll
       for (int i = 0; i < S; ++i)
@@ -244,7 +255,12 @@ __global__ void __launch_bounds__((TL / S) * (TL / S)) contract_gate_kernel(cons
           cfma(th[i][j][1][1], a[i].b, b[j].b);
         }
     }
-    __syncthreads();
+  };
+  fetch(0, va[0], vb[0]);
+  if (DEPTH == 2 && KC < chiM) fetch(KC, va[DEPTH - 1], vb[DEPTH - 1]);
+  for (int r0 = 0; r0 < chiM; r0 += 2 * KC) {
+    step(r0, 0, va[0], vb[0]);
+    if (r0 + KC < chiM) step(r0 + KC, 1, va[DEPTH - 1], vb[DEPTH - 1]);
   }
   CX* X = (CX*)P.X;
 #pragma unroll
