@@ -187,7 +187,15 @@ class ProductList:
     """Products D = op(A) op(B) of any shapes: listed on the host in groups,
     uploaded once, then launched group by group (one launch, or two where a
     group has both kinds).  complex64 products with every dimension >= 32 take
-    the tcgen05 GEMM (3xTF32, float32 accuracy), the rest the SIMT GEMM."""
+    the tcgen05 GEMM (3xTF32, float32 accuracy), the rest the SIMT GEMM, and so
+    do all where the group's 32 x 32 tiles find an SM each: the tensor-core kernel
+    then has a few CTAs, bound by the latency of their K steps.  Measured (us, tcgen05
+    and SIMT): 1 of 256 x 512 x 256, 128 tiles, 17.9 and 12.5; 2 of 256 x 256 x 512, 128
+    tiles, 29.6 and 22.2; 2 of 192 x 384 x 192, 144 tiles, 15.0 and 10.7; 1 of 320 x 640
+    x 320, 200 tiles, 20.9 and 25.1; 4 of 192 x 384 x 192, 288 tiles, 15.1 and 16.4; 4
+    of 256 x 512 x 256, 512 tiles, 18.3 and 38.6."""
+
+    SMS = 152
 
     def __init__(self, dtype, device):
         self.code, self.device = dtype_code(dtype), device
@@ -196,8 +204,9 @@ class ProductList:
 
     def group(self, products):
         """products: (M, N, K, opA, opB, A, lda, B, ldb, D, ldd) with device pointers; returns the group's number."""
-        tc = [p for p in products if self.code == _lib.AGB_C64 and min(p[0], p[1], p[2]) >= 32]
-        rest = [p for p in products if not (self.code == _lib.AGB_C64 and min(p[0], p[1], p[2]) >= 32)]
+        few = sum(-(-p[0] // 32) * -(-p[1] // 32) for p in products) <= self.SMS
+        tc = [] if few or self.code != _lib.AGB_C64 else [p for p in products if min(p[0], p[1], p[2]) >= 32]
+        rest = [p for p in products if not tc or min(p[0], p[1], p[2]) < 32]
         launches = []
         for on, ps in ((1, tc), (0, rest)):
             if ps:
