@@ -4,7 +4,9 @@
 // used by to_left_canonical (adaptive_mps.py:310-339), canonicalize_right_to_left
 // (mps_pytorch.py:123-152) and to_mixed_canonical (adaptive_mps.py:346-385).
 //
-// One CTA (1024 threads = 128 column lanes x 8 row groups) per matrix.  The
+// M N >= 64 x 64: the cluster kernels (qr_blocked.cu, qr_cluster.cu); below, one CTA
+// with everything in shared memory (qr_small_kernel).  qr_kernel, for what neither
+// takes and for agb_qr_noalloc: one CTA (1024 threads = 128 column lanes x 8 row groups).  The
 // matrix op(A) (M x N, op = N or T) is copied into the workspace, reduced with
 // zgeqr2-style reflectors (H_j^H applied from the left), then the thin Q
 // (M x kk, kk = min(M, N)) is formed by applying H_0 ... H_{kk-1} to [I; 0].
@@ -144,6 +146,152 @@ __global__ void __launch_bounds__(1024) qr_kernel(const CX* __restrict__ Ain, in
   }
 }
 
+AGB_DEV float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+AGB_DEV double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// The factorisation of qr_kernel for matrices that fit shared memory, sum for sum:
+// a warp takes four columns, its eight lanes per column the row groups whose partial
+// sums qr_kernel adds in order, so a column's product needs no barrier; in float
+// every warp forms the reflector for itself (double, whose pipe the warps share,
+// leaves it to one), and the thin Q's columns are independent.  One block barrier a
+// column (two in double) instead of eleven, and no round trips to L2.  Bound by the
+// chain of a column (norm, square root, divisions, product, update).
+// 64 x 32: 129 -> 74 us, 32 x 16: 50 -> 28, 90 x 45: 235 -> 129 (complex128, where the
+// FP64 pipe decides: 557 -> 503, 214 -> 142, 1144 -> 1111).
+struct QrSmall {
+  int ld;                     // column stride: 16-lane phases hit distinct banks from 16 rows on
+  size_t w, v, q, total;      // W [N][ld], reflectors and Q [kk][ld]
+};
+AGB_HD QrSmall qr_small_layout(int esz, int M, int N) {
+  QrSmall L;
+  const int kk = M < N ? M : N;
+  L.ld = M < 16 ? (M | 1) : (M + 7) / 16 * 16 + 8;
+  L.w = 0;
+  L.v = (size_t)N * L.ld * esz;
+  L.q = L.v + (size_t)kk * L.ld * esz;
+  L.total = L.q + (size_t)kk * L.ld * esz;
+  return L;
+}
+constexpr int kQrSmallWarps = 16;
+constexpr size_t kQrSmallSmem = 220 * 1024;
+constexpr int kQrSmallCols = 64;  // largest min(M, N) of M N < 64 x 64
+
+template <typename CX>
+__global__ void __launch_bounds__(32 * kQrSmallWarps)
+    qr_small_kernel(const CX* __restrict__ Ain, int M, int N, int transA, CX* Q, CX* R, int trans_out) {
+  typedef typename cx_traits<CX>::R Rt;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const QrSmall L = qr_small_layout(sizeof(CX), M, N);
+  const int ld = L.ld, kk = M < N ? M : N;
+  CX* W = (CX*)(smem_raw + L.w);
+  CX* V = (CX*)(smem_raw + L.v);
+  CX* Z = (CX*)(smem_raw + L.q);
+  __shared__ CX taus[kQrSmallCols], bc;
+  __shared__ Rt diag[kQrSmallCols];
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+  const int rg = lane & 7, cl = lane >> 3;
+  for (int i = tid; i < M * N; i += nt) {
+    const int r = transA ? i % M : i / N, c = transA ? i / M : i % N;
+    W[c * ld + r] = Ain[i];
+  }
+  // (tau, scale of v) of column j; every lane ends with them
+  auto reflect = [&](int j, CX& t, CX& sc) {
+    const CX* col = W + j * ld;
+    Rt kept = 0;
+    for (int w = 0; j + 1 + 32 * w < M && w < 32; ++w) {
+      Rt p = 0;
+      for (int r = j + 1 + 32 * w + lane; r < M; r += 1024) p += cabs2(col[r]);
+      p = warp_sum(p);
+      if (lane == w) kept = p;
+    }
+    const Rt xn2 = warp_sum(kept);
+    const CX alpha = col[j];
+    Rt beta;
+    t = sc = czero<CX>();
+    if (xn2 == Rt(0) && alpha.y == Rt(0)) {
+      beta = alpha.x;
+    } else {
+      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
+      t = mk<CX>((beta - alpha.x) / beta, -alpha.y / beta);
+      sc = cinv(csub(alpha, mk<CX>(beta, 0)));
+    }
+    if (wid == j % nw || sizeof(Rt) == 8) {
+      if (lane == 0) {
+        taus[j] = t;
+        diag[j] = beta;
+      }
+    }
+  };
+  // y (column c of Y) -= v scale(v^H y); v below row j as `vec` gives it, 1 in row j.
+  // `scale` spells out which of its products are fused, as qr_kernel rounds them.
+  auto apply = [&](CX* Y, int c, bool on, int j, auto scale, auto vec) {
+    CX acc = czero<CX>();
+    CX* y = Y + (on ? c : 0) * ld;
+    if (on)
+      for (int r = j + rg; r < M; r += 8) cfmac(acc, r == j ? mk<CX>(1, 0) : vec(r), y[r]);
+    CX w = czero<CX>();
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+      w = cadd(w, mk<CX>(__shfl_sync(0xffffffffu, acc.x, g, 8), __shfl_sync(0xffffffffu, acc.y, g, 8)));
+    const CX tw = scale(w);
+    if (on)
+      for (int r = j + rg; r < M; r += 8) y[r] = csub(y[r], cmul(r == j ? mk<CX>(1, 0) : vec(r), tw));
+  };
+  __syncthreads();
+  for (int j = 0; j < kk; ++j) {
+    CX t, sc;
+    if (sizeof(Rt) == 4) {
+      reflect(j, t, sc);
+    } else {
+      if (wid == 0) {
+        reflect(j, t, sc);
+        if (lane == 0) bc = sc;
+      }
+      __syncthreads();
+      t = taus[j];
+      sc = bc;
+    }
+    const CX* col = W + j * ld;
+    if (wid == j % nw)
+      for (int r = j + 1 + lane; r < M; r += 32) V[j * ld + r] = cmul(col[r], sc);
+    if (t.x != Rt(0) || t.y != Rt(0)) {
+      auto scale = [&](CX w) {  // conj(tau) w
+        return mk<CX>(fma(t.y, w.y, mul_rn(t.x, w.x)), fma(t.x, w.y, -mul_rn(t.y, w.x)));
+      };
+      for (int c0 = (j + 1) / 4 * 4 + 4 * ((wid - (j + 1) / 4 % nw + nw) % nw); c0 < N; c0 += 4 * nw) {
+        const int c = c0 + cl;
+        apply(W, c, c > j && c < N, j, scale, [&](int r) { return cmul(col[r], sc); });
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < kk * N; i += nt) {
+    const int r = trans_out ? i % kk : i / N, c = trans_out ? i / kk : i % N;
+    R[i] = c > r ? W[c * ld + r] : c == r ? mk<CX>(diag[r], 0) : czero<CX>();
+  }
+  // Q = H_0 ... H_{kk-1} [I; 0], each warp on its own columns
+  for (int c0 = 4 * wid; c0 < kk; c0 += 4 * nw) {
+    const int c = c0 + cl;
+    if (c < kk)
+      for (int r = rg; r < M; r += 8) Z[c * ld + r] = r == c ? mk<CX>(1, 0) : czero<CX>();
+    __syncwarp();
+    for (int j = min(kk - 1, c0 + 3); j >= 0; --j) {
+      const CX t = taus[j];
+      if (t.x == Rt(0) && t.y == Rt(0)) continue;
+      auto scale = [&](CX w) {  // tau w
+        return mk<CX>(fma(t.x, w.x, -mul_rn(t.y, w.y)), fma(t.x, w.y, mul_rn(t.y, w.x)));
+      };
+      apply(Z, c, c >= j && c < kk, j, scale, [&](int r) { return V[j * ld + r]; });
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < M * kk; i += nt) {
+    const int c = trans_out ? i / M : i % kk, r = trans_out ? i % M : i / kk;
+    Q[i] = Z[c * ld + r];
+  }
+}
+
 }  // namespace
 
 // working copy of op(A), tau, column-major Q (single-CTA and unblocked cluster kernels)
@@ -189,6 +337,19 @@ extern "C" int agb_qr(int dtype, const void* A, int M, int N, int transA, void* 
                        : launch_qr_cluster<double2>((const double2*)A, M, N, transA, (double2*)Q, (double2*)R,
                                                     trans_out, (double2*)Qw, s);
     if (rc == AGB_OK) return AGB_OK;
+  } else if (qr_small_layout(esz, M, N).total <= kQrSmallSmem) {
+    const size_t sm = qr_small_layout(esz, M, N).total;
+    const int nw = (N + 3) / 4 < kQrSmallWarps ? (N + 3) / 4 : kQrSmallWarps;
+    if (dtype == AGB_C64) {
+      if (agb_smem_optin(qr_small_kernel<float2>, sm) != cudaSuccess) return AGB_ERR_CUDA;
+      qr_small_kernel<float2><<<1, 32 * nw, sm, s>>>((const float2*)A, M, N, transA, (float2*)Q, (float2*)R, trans_out);
+    } else {
+      if (agb_smem_optin(qr_small_kernel<double2>, sm) != cudaSuccess) return AGB_ERR_CUDA;
+      qr_small_kernel<double2><<<1, 32 * nw, sm, s>>>((const double2*)A, M, N, transA, (double2*)Q, (double2*)R,
+                                                      trans_out);
+    }
+    AGB_CHECK_LAUNCH();
+    return AGB_OK;
   }
   if (dtype == AGB_C64) {
     if (agb_smem_optin(qr_kernel<float2>, smem) != cudaSuccess) return AGB_ERR_CUDA;

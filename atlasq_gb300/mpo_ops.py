@@ -180,7 +180,8 @@ def expectation_value(mpo: MPO, mps, use_gpu_optimized: bool = True) -> complex:
     wsp, wsn, status = ptr(ws), ws.numel(), ptr(ops._tc_status_word(dev))
 
     def product(opA, m, nn, k, A, lda, B, ldb, C):  # the norm's: tensor cores as in ProductList
-        if code == _lib.AGB_C64 and min(m, nn, k) >= 32:
+        few = -(-m // 32) * -(-nn // 32) <= ops.ProductList.SMS
+        if code == _lib.AGB_C64 and min(m, nn, k) >= 32 and not few:
             rc = lib.agb_cgemm_tc_async(opA, b"N", 1, m, nn, k, A, lda, 0, B, ldb, 0, C, nn, 0, 1.0, 0.0, 0.0, 0.0,
                                         wsp, wsn, status, stream)
         else:
