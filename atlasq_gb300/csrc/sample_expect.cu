@@ -18,44 +18,84 @@
 
 namespace {
 
-template <typename CX>
-__global__ void sample_site_kernel(const CX* __restrict__ temp, int shots, int chiR, int site,
-                                   uint64_t seed, uint64_t shot_offset, int64_t* __restrict__ bits,
-                                   CX* __restrict__ Lnew, double* __restrict__ pz_out) {
-  const int lane = threadIdx.x & 31;
-  const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (s >= shots) return;
+// A warp per shot, kSampleShots shots per CTA.  The row is read once, into registers,
+// all of its loads in flight, where a lane's share is at most K elements a half (K = 0:
+// any length, read again for the output).  The decisions of a CTA's shots (two dozen
+// FP64 instructions, whatever the number of active lanes, at 16 cycles of the SM's
+// pipe) are taken together by one warp: by each shot's own warp they were 20 us for
+// 16 384 shots, more than the traffic.  16 384 shots: chi 256
+// 25 -> 20 us (5.1 TB/s, from L2), chi 64 22.5 -> 7.4.
+constexpr int kSampleShots = 16;
+template <typename CX, int K>
+__global__ void __launch_bounds__(32 * kSampleShots) sample_site_kernel(const CX* __restrict__ temp, int shots, int chiR, int site,
+                                                          uint64_t seed, uint64_t shot_offset,
+                                                          int64_t* __restrict__ bits, CX* __restrict__ Lnew,
+                                                          double* __restrict__ pz_out) {
   typedef typename cx_traits<CX>::R R;
-  const CX* row = temp + (int64_t)s * 2 * chiR;
-  // both probabilities to double accuracy on the FP32 pipe; the decision
-  // (double division, Philox) runs once per shot, in lane 0
+  __shared__ __align__(16) unsigned char sum_raw[2 * kSampleShots * sizeof(SumAcc<R>)];
+  SumAcc<R>* sums = (SumAcc<R>*)sum_raw;  // [2][kSampleShots]
+  __shared__ int outcome[kSampleShots];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int s0 = blockIdx.x * kSampleShots, s = s0 + wid;
+  const bool on = s < shots;
+  const CX* row = temp + (int64_t)(on ? s : 0) * 2 * chiR;
+  // both probabilities to double accuracy on the FP32 pipe
   SumAcc<R> a0, a1;
-  for (int c = lane; c < chiR; c += 32) {
-    a0.add(cabs2(row[c]));
-    a1.add(cabs2(row[chiR + c]));
+  CX v0[K ? K : 1], v1[K ? K : 1];
+  if (K) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = lane + 32 * k;
+      v0[k] = c < chiR ? row[c] : czero<CX>();
+      v1[k] = c < chiR ? row[chiR + c] : czero<CX>();
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (lane + 32 * k < chiR) {
+        a0.add(cabs2(v0[k]));
+        a1.add(cabs2(v1[k]));
+      }
+  } else {
+    for (int c = lane; c < chiR; c += 32) {
+      a0.add(cabs2(row[c]));
+      a1.add(cabs2(row[chiR + c]));
+    }
   }
   a0.warp_reduce();
   a1.warp_reduce();
-  int outc = 0;
   if (lane == 0) {
-    const double p0 = a0.value() + 1e-15, p1 = a1.value() + 1e-15;
+    sums[wid] = a0;
+    sums[kSampleShots + wid] = a1;
+  }
+  __syncthreads();
+  if (wid == 0 && lane < kSampleShots && s0 + lane < shots) {
+    const int t = s0 + lane;
+    const double p0 = sums[lane].value() + 1e-15, p1 = sums[kSampleShots + lane].value() + 1e-15;
     const double pz = p0 / (p0 + p1);
-    const uint64_t shot = shot_offset + (uint64_t)s;
+    const uint64_t shot = shot_offset + (uint64_t)t;
     const philox_out o = philox4x32_10((uint32_t)shot, (uint32_t)(shot >> 32), (uint32_t)site, 0u,
                                        (uint32_t)seed, (uint32_t)(seed >> 32));
     const double u = (double)(o.x >> 8) * (1.0 / 16777216.0);
-    outc = (u >= pz) ? 1 : 0;
-    bits[s] = (bits[s] << 1) | outc;
-    if (pz_out) pz_out[s] = pz;
+    const int outc = (u >= pz) ? 1 : 0;
+    bits[t] = (bits[t] << 1) | outc;
+    if (pz_out) pz_out[t] = pz;
+    outcome[lane] = outc;
   }
-  outc = __shfl_sync(0xffffffffu, outc, 0);
-  if (Lnew) {
-    const CX* src = row + outc * chiR;
-    for (int c = lane; c < chiR; c += 32) Lnew[(int64_t)s * chiR + c] = src[c];
+  __syncthreads();
+  const int outc = outcome[wid];
+  if (Lnew && on) {
+    CX* dst = Lnew + (int64_t)s * chiR;
+    if (K) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < chiR) dst[lane + 32 * k] = outc ? v1[k] : v0[k];
+    } else {
+      const CX* src = row + outc * chiR;
+      for (int c = lane; c < chiR; c += 32) dst[c] = src[c];
+    }
   }
 }
 
-// N[R][a][t][B] = sum_{L,s} W[L][s][t][R] * M[L][a][s][B]
 template <typename CX>
 __global__ void mpo_mix_kernel(const CX* __restrict__ M, const CX* __restrict__ W, CX* __restrict__ N,
                                int Lw, int Rw, int chiA, int chiB) {
@@ -179,15 +219,21 @@ extern "C" int agb_sample_site(int dtype, const void* temp, int shots, int chiR,
   if (dtype != AGB_C64 && dtype != AGB_C128) return AGB_ERR_ARG;
   if (shots < 0 || chiR <= 0 || !temp || !bits) return AGB_ERR_ARG;
   if (shots == 0) return AGB_OK;
-  const int wpb = 8;
-  dim3 grid((shots + wpb - 1) / wpb);
+  const dim3 grid((shots + kSampleShots - 1) / kSampleShots);
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == AGB_C64)
-    sample_site_kernel<float2><<<grid, 32 * wpb, 0, s>>>((const float2*)temp, shots, chiR, site, seed,
-                                                         shot_offset, bits, (float2*)Lnew, pz_out);
-  else
-    sample_site_kernel<double2><<<grid, 32 * wpb, 0, s>>>((const double2*)temp, shots, chiR, site, seed,
-                                                          shot_offset, bits, (double2*)Lnew, pz_out);
+  auto run = [&](auto kern, auto cx) {
+    typedef decltype(cx) CX;
+    kern<<<grid, 32 * kSampleShots, 0, s>>>((const CX*)temp, shots, chiR, site, seed, shot_offset, bits, (CX*)Lnew, pz_out);
+  };
+  if (dtype == AGB_C64) {
+    if (chiR <= 64) run(sample_site_kernel<float2, 2>, float2());
+    else if (chiR <= 128) run(sample_site_kernel<float2, 4>, float2());
+    else if (chiR <= 256) run(sample_site_kernel<float2, 8>, float2());
+    else run(sample_site_kernel<float2, 0>, float2());
+  } else {
+    if (chiR <= 128) run(sample_site_kernel<double2, 4>, double2());
+    else run(sample_site_kernel<double2, 0>, double2());
+  }
   AGB_CHECK_LAUNCH();
   return AGB_OK;
 }
