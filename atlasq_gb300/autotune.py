@@ -1,8 +1,9 @@
 """Autotuning of the launch shapes the two-site pipeline uses.
 
 The Householder tridiagonalisation (the eigensolver's first and longest stage)
-runs one thread-block cluster per Gram matrix, keeping the packed matrix in the
-cluster's distributed shared memory.  How many CTAs a cluster should have
+runs one thread-block cluster per Gram matrix, keeping the matrix on chip:
+complex64 in the cluster's registers and shared memory, complex128 packed in
+its distributed shared memory.  How many CTAs a cluster should have
 depends on the matrix size and on how many problems share the GPU in one
 launch (a 512 x 512 problem alone wants every SM it can get; twenty of them
 want the cluster that just fits).  ``tune_tridiag`` times each admissible

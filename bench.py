@@ -576,25 +576,25 @@ def main():
     roof.update({"kernel": dom, "peak_source": src, "stage_ms_per_step": {k: round(v, 3) for k, v in stage_ms.items()},
                  "algorithmic_flops_per_step": wf, "algorithmic_bytes_per_step": wb})
     if dom == "tridiag":
-        # The Householder reduction keeps each matrix in the shared memory of an
-        # 8-CTA cluster, so HBM is not what limits it: one launch per layer runs
-        # n - 1 dependent column steps, each a row pass and a column pass issued
-        # by one 16-warp CTA per SM (the packed rows fill its shared memory).
+        # The Householder reduction keeps each matrix in the registers and shared
+        # memory of a cluster, so HBM is not what limits it: one launch per layer
+        # runs n - 1 dependent column steps, each a pass over the own rows and two
+        # exchanges, by one 8-warp CTA per SM (its rows fill the register file).
         # Its FP32 rate is reported beside the HBM fraction of the contract.
         fp32_peak = 152 * 128 * 2 * (clocks.get("sm_max_mhz") or 2070.0) / 1e6  # TFLOP/s, SIMT FMA
-        roof["limiter"] = ("instruction issue: n - 1 dependent column steps of ~960 instructions per warp at "
-                           "~31% issue activity, one 16-warp CTA per SM (not HBM)")
+        roof["limiter"] = ("latency: n - 1 dependent column steps (pass over the own rows, norm, reflector, two "
+                           "exchanges) at ~35% issue activity, one 8-warp CTA per SM (not HBM)")
         roof["fp32_simt"] = {"achieved_tflops": wf / t_dom / 1e12 if t_dom > 0 else 0.0,
                              "peak_tflops": fp32_peak,
                              "frac": (wf / t_dom / 1e12) / fp32_peak if t_dom > 0 else 0.0}
         # DRAM bytes of ONE launch (one saturated layer: 20 Gram matrices of
-        # 512 x 512) from an ncu capture of this kernel on this workload: read
-        # 14 264 064 B, written 0 B, against that launch's 20 x 2 n^2 x 8 B =
-        # 83 886 080 algorithmic bytes (the rest is served from L2, where the
+        # 512 x 512) from an ncu capture of this kernel on 20 matrices of that
+        # size: read 21 728 768 B, written 0 B, against that launch's 20 x 2 n^2 x
+        # 8 B = 83 886 080 algorithmic bytes (the rest is served from L2, where the
         # Gram GEMM left it).  Per launch, not per step.
-        roof["traffic"] = 14264064
+        roof["traffic"] = 21728768
         roof["traffic_per_launch"] = {"matrices": 20, "n": 512, "algorithmic_bytes": 20 * 2 * 512 * 512 * 8,
-                                      "dram_bytes": 14264064,
+                                      "dram_bytes": 21728768,
                                       "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch"}
 
     line = {"metric": METRIC, "value": value, "unit": "gates/s", "n_gpus": ws, "steps": args.steps,
@@ -605,7 +605,7 @@ def main():
                 "l2": "flushed between timed steps (2x L2 write)",
                 "precision": "complex64; Gram / X.V / polish GEMMs on tcgen05 (3xTF32), FP32 eigensolver",
                 "tridiagonalisation": ("two-stage (band reduction + bulge chasing)" if args.two_stage else
-                                       "one-stage, matrix in cluster shared memory"),
+                                       "one-stage, matrix in cluster registers and shared memory"),
                 "execution": "device-resident (no host sync between batches)" if RESIDENT else
                              "host-synchronised (ranks read back after every batch)"},
             "clocks": clocks, "gpu_launches": launches, "e2e": e2e, "roofline": roof, "other_mode": other_mode}
