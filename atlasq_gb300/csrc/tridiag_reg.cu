@@ -23,7 +23,8 @@
 //   C. that CTA adds the V partials, scales by tau and sends its slice of p and
 //      of row j + 1 to every CTA.
 // The exchanges are remote stores that count their bytes on the receiver's
-// mbarrier (st.async), so a step has no cluster barrier and no fence.  A matrix
+// mbarrier (st.async), so a step has no cluster barrier and no fence; every CTA
+// waits for a word of every other on both barriers (tridiag_exchange.cuh).  A matrix
 // whose rows fit one CTA (n <= 128) exchanges through its own shared memory.
 //
 // What bounds it: the FP32 pipe in pass B (a third of 12 n^2 / C FMAs per step on
@@ -38,11 +39,13 @@
 #include "heevd.cuh"
 #include "householder.cuh"
 #include "prof.cuh"
+#include "tridiag_exchange.cuh"
 
 namespace {
 
 constexpr int NT = 256;
 constexpr int NW = NT / 32;
+static_assert(NW == exchange::kWarps, "words of the exchange");
 constexpr int UB = 4;        // register rows per branch of the pass
 constexpr int PAD = UB - 1;  // row-factor entries in front (the slots below an owner's first row)
 
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(NT, 1)
   }
   const int base = nr - RR;  // slot of register row 0 (may be negative)
   const int ngm = (base > 0 ? base : 0) - nsm;
-  const int S = ((n + Ce - 1) / Ce + CPT - 1) / CPT * CPT;  // columns of a CTA's slice
+  const int S = exchange::slice(n, Ce, CPT);  // columns of a CTA's slice
 
   // ---- scale by the largest diagonal magnitude (every CTA reads the diagonal)
   float mx = 0;
@@ -264,12 +267,11 @@ __global__ void __launch_bounds__(NT, 1)
   const uint32_t part_addr = peer_addr(smem_u32(part + (size_t)o * S + (c0 - dq * S)), dq);
   const uint32_t row_addr = peer_addr(smem_u32(rowsl + (c0 - dq * S)), dq);
   const uint32_t part_bar = peer_addr(bar1, dq);
-  // the warp's share of v^H A v goes to CTA wid % Ce, which gets npw from every CTA
-  const int npw = (NW + Ce - 1) / Ce;
-  const uint32_t dot_addr = peer_addr(smem_u32(wdots + q * npw + wid / Ce), wid % Ce);
-  const uint32_t dot_bar = peer_addr(bar1, wid % Ce);
-  const int ndot = q < NW ? (NW - q + Ce - 1) / Ce * Ce : 0;  // shares that arrive here
-  const int nslice = min(n, q * S + S);                      // end of the own slice
+  // the warp's share of v^H A v, and a zero for a CTA that gets no share
+  const int dd = exchange::dot_dest(wid, Ce);
+  const uint32_t dot_addr = peer_addr(smem_u32(wdots + q * exchange::dot_pitch(Ce) + wid / Ce), dd);
+  const uint32_t dot_bar = peer_addr(bar1, dd);
+  const int dz = exchange::zero_dest(wid, Ce);
   int fac[CPT];   // row-factor entry of row c when this owner holds it, else an unused one
   float2 v[CPT];  // own columns of v (step j-1 until A, then step j)
   float2 w[CPT];  // own columns of w of step j-1
@@ -534,14 +536,12 @@ __global__ void __launch_bounds__(NT, 1)
     if (lane == 0) {
       if (Ce == 1) wdots[wid] = sd;
       else send(dot_addr, dot_bar, sd);
+      if (dz >= 0) send(peer_addr(smem_u32(wdots + q), dz), peer_addr(bar1, dz), 0.f);
     }
     // off the exchange's critical path: bytes to expect, the stored reflector, the next row
     if (tid == 0 && Ce > 1) {
-      // pairs of columns of the own slice still in use (CPT at a time)
-      const int f0 = max(q * S, (j + 1) / CPT * CPT);
-      const int sl = nslice > f0 ? (nslice - f0 + CPT - 1) / CPT : 0;
-      bar_expect(bar1, (uint32_t)(sl * (V + 1) * CPT * 8 + ndot * 4));
-      bar_expect(bar2, (uint32_t)((n - 1 - j) * 16 + Ce * 4));
+      bar_expect(bar1, (uint32_t)exchange::bytes1(n, Ce, V, CPT, q, j));
+      bar_expect(bar2, (uint32_t)exchange::bytes2(n, Ce, j));
     }
     if (o == 0 && j - c0 >= 0 && j - c0 < CPT) dg[j] = dj;
     if (turn == q && g == 0) {
@@ -578,14 +578,15 @@ __global__ void __launch_bounds__(NT, 1)
     }
     if (!bar_wait(bar1, j & 1)) ok = false;
     // ---------------- C: reduce the own column slice; p and row j+1 of it to every CTA
-    if (wid == NW - 1 && lane < Ce) {
+    if (wid == NW - 1) {
       float s = 0.f;
 #pragma unroll
       for (int i = 0; i < 16; i += 4) {
         const float4 z = *(const float4*)(wdots + i);
         s += (z.x + z.y) + (z.z + z.w);
       }
-      send(peer_addr(smem_u32(dots + q), lane), peer_addr(bar2, lane), s);
+      __syncwarp();  // the first word sent lets a peer write the next step's shares
+      if (lane < Ce) send(peer_addr(smem_u32(dots + q), lane), peer_addr(bar2, lane), s);
     }
     for (int cl = tid; cl < S; cl += NT) {
       const int c = q * S + cl;
