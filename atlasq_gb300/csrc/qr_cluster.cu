@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(QRC_THREADS, 1)
     CX* col = cols + (size_t)lc * M;
     for (int r = lane; r < M; r += 32) col[r] = transA ? Ain[(int64_t)c * M + r] : Ain[(int64_t)r * N + c];
   }
-  __syncthreads();
+  cluster.sync();  // every CTA has started: its shared memory may be written from here on
   // ---- factorisation
   for (int j = 0; j < kk; ++j) {
     const int owner = j % C, b = j & 1;

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(512, 1) tridiag_cluster_kernel(const HeevdProb
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) red[wid] = mx;
-  __syncthreads();
+  cluster.sync();  // every CTA has started: its shared memory may be written from here on
   if (tid == 0) {
     R m = 0;
     for (int i = 0; i < nw; ++i) m = fmax(m, red[i]);

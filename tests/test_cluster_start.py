@@ -1,0 +1,30 @@
+"""Distributed shared memory may be touched only once every CTA of the cluster has
+started: in each kernel a cluster barrier stands before the first access to a peer's
+shared memory (read from the source; a run cannot show the order it happened to have)."""
+import pathlib
+import re
+
+import pytest
+
+CSRC = pathlib.Path(__file__).resolve().parents[1] / "atlasq_gb300" / "csrc"
+REMOTE = re.compile(r"map_shared_rank\(|\bsend\(")
+BARRIER = re.compile(r"cluster\.sync\(\)|cluster_barrier\(\)")
+
+
+def _kernels():
+    for f in sorted(CSRC.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", f.read_text())
+        for body in text.split("__global__")[1:]:
+            if REMOTE.search(body):
+                yield f.name, re.search(r"\w+_kernel(?=\()", body).group(0), body
+
+
+@pytest.mark.parametrize("name,kernel,body", [pytest.param(*k, id=f"{k[0]}-{k[1]}") for k in _kernels()])
+def test_cluster_barrier_before_the_first_remote_access(name, kernel, body):
+    first, barrier = REMOTE.search(body).start(), BARRIER.search(body)
+    assert barrier and barrier.start() < first, f"{name}: {kernel}"
+
+
+def test_the_cluster_kernels_are_found():
+    assert {n for n, _, _ in _kernels()} >= {"tridiag_reg.cu", "tridiag_cluster.cu", "tridiag_2stage.cu",
+                                             "qr_cluster.cu"}
