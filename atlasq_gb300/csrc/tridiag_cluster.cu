@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(512, 1) tridiag_cluster_kernel(const HeevdProb
   }
   __syncthreads();
   if (n == 1) {
-    if (tid == 0) {
+    if (q == 0 && tid == 0) {
       d[0] = rowp(0)[0].x;
       e[0] = 0;
       tau[0] = czero<CX>();
