@@ -150,6 +150,28 @@ class MPOBuilder:
         return MPO(sites, n_sites)
 
 
+def _chain(tensors, right=1):
+    """Site tensors of an open chain, contiguous and of the first one's dtype: the
+    kernels get pointers and bonds, so every shape is checked before one is taken.
+    ``right``: the last bond (None: any)."""
+    bond, dev = 1, tensors[0].device
+    for i, A in enumerate(tensors):
+        if A.dim() != 3 or A.shape[1] != 2 or min(A.shape) < 1:
+            raise ValueError(f"site {i}: expected a tensor [left, 2, right], got {tuple(A.shape)}")
+        if A.shape[0] != bond:
+            raise ValueError(f"site {i}: inner dimension mismatch {bond} vs {A.shape[0]}")
+        if A.device != dev:
+            raise ValueError(f"site {i} is on {A.device}, site 0 on {dev}")
+        bond = A.shape[2]
+    if right is not None and bond != right:
+        raise ValueError(f"site {len(tensors) - 1}: right boundary bond {bond} instead of {right}")
+    dtype_code(tensors[0].dtype)
+    if dev.type != "cuda":
+        raise ValueError(f"site tensors are on {dev}, expected a CUDA device")
+    dt = tensors[0].dtype
+    return [(A if A.dtype == dt else A.to(dt)).contiguous() for A in tensors]
+
+
 @torch.no_grad()
 def expectation_value(mpo: MPO, mps, use_gpu_optimized: bool = True) -> complex:
     """mpo_ops.py:1085-1169 (standard MPO contraction path).  Per site, with E
@@ -159,12 +181,19 @@ def expectation_value(mpo: MPO, mps, use_gpu_optimized: bool = True) -> complex:
     lib = _lib.load()
     n = mpo.n_sites
     assert n == mps.num_qubits
-    tensors = [t.contiguous() for t in mps.tensors]
+    tensors, Ws = list(mps.tensors), list(mpo.tensors)
+    if len(tensors) < n or len(Ws) < n:
+        raise IndexError(f"{n} sites, but {len(tensors)} site tensors and {len(Ws)} operator tensors")
+    Ws = [_as_site(W, i) for i, W in enumerate(Ws[:n])]
+    lefts = [1] + [W.shape[3] for W in Ws[:-1]]  # channels that arrive at each site
+    for i, (W, left) in enumerate(zip(Ws, lefts)):
+        if W.shape[0] < left or W.shape[3] < 1:
+            raise ValueError(f"MPO site {i}: {left} channels arrive at {W.shape[0]}, {W.shape[3]} leave")
+    tensors = _chain(tensors[:n], right=None)
     dt = tensors[0].dtype
     dev = tensors[0].device
     code, stream = dtype_code(dt), stream_ptr(dev)
-    tensors = [t if t.dtype == dt else t.to(dt).contiguous() for t in tensors]
-    Ws = [W.to(dtype=dt, device=dev).contiguous() for W in mpo.tensors]
+    Ws = [W.to(dtype=dt, device=dev).contiguous() for W in Ws]
     big = max(max(W.shape[0], W.shape[3], 1) * t.numel() for W, t in zip(Ws, tensors))
     env = max(W.shape[3] * t.shape[2] ** 2 for W, t in zip(Ws, tensors))
     # E (two), the products and their mix, then the same for the norm
@@ -191,7 +220,7 @@ def expectation_value(mpo: MPO, mps, use_gpu_optimized: bool = True) -> complex:
 
     for i, (A, W) in enumerate(zip(tensors, Ws)):
         l, _, r = A.shape
-        Lw, Rw = W.shape[0], W.shape[3]
+        Lw, Rw = lefts[i], W.shape[3]
         p, cur, nxt = A.data_ptr(), i & 1, 1 - (i & 1)
         check(lib.agb_cgemm_batched(code, b"N", b"N", Lw, l, 2 * r, l, E[cur], l, l * l, p, 2 * r, 0, M, 2 * r,
                                     2 * l * r, 1.0, 0.0, 0.0, 0.0, stream), "expectation_value")
@@ -234,8 +263,8 @@ def environments(mps):
     environments Renv[i] (after site i-1, stored as [ket, bra]) for i = 0..n.
     The two sweeps do not depend on each other: site s of the left one and site
     n-1-s of the right one share their launches (two per step)."""
-    dt = mps.tensors[0].dtype
-    tensors = [t.contiguous() if t.dtype == dt else t.to(dt).contiguous() for t in mps.tensors]
+    tensors = _chain(list(mps.tensors))
+    dt = tensors[0].dtype
     dev = tensors[0].device
     n = len(tensors)
     d = [t.shape[0] for t in tensors] + [tensors[-1].shape[2]]
@@ -302,6 +331,8 @@ def _local_chunk(tensors, Lenv, Renv, observables, dt, dev, norm):
     spans = []
     for obs in observables:
         sites = sorted(obs)
+        if sites[0] < 0 or sites[-1] >= len(tensors):
+            raise IndexError(f"observable on sites {sites} of a chain of {len(tensors)}")
         spans.append((sites[0], sites[-1]))
     eye = torch.eye(2, dtype=dt)
     mats, rounds = [], []  # rounds: per round [(observable, site)]
@@ -310,9 +341,9 @@ def _local_chunk(tensors, Lenv, Renv, observables, dt, dev, norm):
         mats += [observables[k].get(s, eye) for k, s in act]
         rounds.append(act)
     if all(m.device.type == "cpu" for m in mats):
-        W = torch.stack([m.to(dt) for m in mats]).to(dev) if mats else None
+        W = torch.stack([m.to(dt).reshape(2, 2) for m in mats]).to(dev) if mats else None
     else:
-        W = torch.stack([m.to(device=dev, dtype=dt) for m in mats])
+        W = torch.stack([m.to(device=dev, dtype=dt).reshape(2, 2) for m in mats])
     big = max([sum(shapes[s][0] * 2 * shapes[s][1] for _, s in act) for act in rounds], default=0)
     env = max([sum(shapes[s][1] ** 2 for _, s in act) for act in rounds], default=0)
     buf = torch.empty(2 * big + 2 * env, dtype=dt, device=dev)
