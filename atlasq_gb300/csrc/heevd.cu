@@ -195,13 +195,15 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(const HeevdProb* __restri
 // a relative change of a few ulp in d_i - x and e_{i-1}^2, like the pivots q_i = p_i /
 // p_{i-1} of the LDL^T form, whose division is most of its chain (FP64 ~880 cycles
 // a step, float ~50).  A zero p_i counts as a small negative pivot, so the count and
-// the recurrence see the same sign.  The pair is rescaled by a power of two every U
-// steps (8 in double, 4 in float): |d_i - x| and e^2 are below 8 after the scaling of
-// H, and factors below the range's U-th root only occur for |x| far below the
-// tolerance.
+// the recurrence see the same sign.
+// Range: the caller scales T so that the largest |d_i|, |e_i| is in [1, 4).  A step then
+// grows the pair (p_i, p_{i-1}) by at most 2^5, and it is rescaled by a power of two every
+// U steps.  It may shrink by any factor (d_i - x and e_i both small): where the U steps
+// took it below `low`, they are repeated with a rescaling each.  In a pair that stayed above,
+// an underflow changes d_i or e_i by less than 2^-32 (float; 2^-300 double).
 AGB_DEV unsigned sign_bits(float a, float b) { return (unsigned)(__float_as_int(a) ^ __float_as_int(b)) >> 31; }
 AGB_DEV unsigned sign_bits(double a, double b) { return (unsigned)(__double2hiint(a) ^ __double2hiint(b)) >> 31; }
-// 2^-exponent of the larger of a and b
+// 2^-exponent of the larger of a and b, which is below 2^126 (2^1022)
 AGB_DEV float pair_scale(float a, float b) {
   const int h = max(__float_as_int(a) & 0x7f800000, __float_as_int(b) & 0x7f800000);
   return __int_as_float(0x7f000000 - h);
@@ -210,10 +212,22 @@ AGB_DEV double pair_scale(double a, double b) {
   const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
   return __hiloint2double(0x7fe00000 - h, 0);
 }
+// 2^e with 2^e <= a < 2^(e+1) (e kept where 2^-e is a normal number too), and 2^-e
+AGB_DEV void power_of(float a, float& p, float& inv) {
+  const int h = min(max(__float_as_int(a) & 0x7f800000, 0x00800000), 0x7e800000);
+  p = __int_as_float(h);
+  inv = __int_as_float(0x7f000000 - h);
+}
+AGB_DEV void power_of(double a, double& p, double& inv) {
+  const int h = min(max(__double2hiint(a) & 0x7ff00000, 0x00100000), 0x7fd00000);
+  p = __hiloint2double(h, 0);
+  inv = __hiloint2double(0x7fe00000 - h, 0);
+}
 template <typename R>
 AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
   constexpr int U = sizeof(R) == 8 ? 8 : 4;
   constexpr R tiny = sizeof(R) == 8 ? R(0x1p-200) : R(0x1p-60f);
+  constexpr R low = sizeof(R) == 8 ? R(0x1p-400) : R(0x1p-60f);
   R p2 = 1, p1 = d[0] - x;
   if (p1 == R(0)) p1 = -tiny;
   int cnt = p1 < R(0);
@@ -224,15 +238,41 @@ AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
     p2 = p1;
     p1 = p;
   };
-  int i = 1;
-  for (; i + U <= n; i += U) {
-#pragma unroll
-    for (int k = 0; k < U; ++k) step(i + k);
+  auto rescale = [&]() {
     const R f = pair_scale(p1, p2);
     p1 *= f;
     p2 *= f;
+  };
+  auto sure_step = [&](int i) {
+    rescale();
+    const R p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
+    if (p == R(0)) {
+      ++cnt;
+      p2 = copysign(R(1), p1);
+      p1 = -copysign(tiny, p1);
+    } else {
+      cnt += (int)sign_bits(p, p1);
+      p2 = p1;
+      p1 = p;
+    }
+  };
+  int i = 1;
+  for (; i + U <= n; i += U) {
+    const R b1 = p1, b2 = p2;
+    const int before = cnt;
+#pragma unroll
+    for (int k = 0; k < U; ++k) step(i + k);
+    if (!(fmax(fabs(p1), fabs(p2)) >= low)) {
+      p1 = b1;
+      p2 = b2;
+      cnt = before;
+#pragma unroll 1
+      for (int k = 0; k < U; ++k) sure_step(i + k);
+    }
+    rescale();
   }
-  for (; i < n; ++i) step(i);
+#pragma unroll 1
+  for (; i < n; ++i) sure_step(i);
   return cnt;
 }
 
@@ -248,21 +288,23 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* d = (R*)smem_raw;
   R* e2 = d + n;
-  __shared__ R glim[2];
+  __shared__ R lim[4];  // Gershgorin interval of the scaled T; the scale and its inverse
   const R* dg = (const R*)P.d;
   const R* eg = (const R*)P.e;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    d[i] = dg[i];
-    e2[i] = (i < n - 1) ? eg[i] * eg[i] : R(0);
-  }
-  __syncthreads();
-  // Gershgorin interval (min and max do not depend on the order)
   if (threadIdx.x < 32) {
-    R gl = d[0], gu = d[0];
+    // min and max do not depend on the order
+    R big = 0;
+    for (int i = threadIdx.x; i < n; i += 32)
+      big = fmax(big, fmax(fabs(dg[i]), i < n - 1 ? fabs(eg[i]) : R(0)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+    R unit, s;
+    power_of(big, unit, s);
+    R gl = dg[0] * s, gu = gl;
     for (int i = threadIdx.x; i < n; i += 32) {
-      const R r = (i > 0 ? fabs(eg[i - 1]) : R(0)) + (i < n - 1 ? fabs(eg[i]) : R(0));
-      gl = fmin(gl, d[i] - r);
-      gu = fmax(gu, d[i] + r);
+      const R r = (i > 0 ? fabs(eg[i - 1] * s) : R(0)) + (i < n - 1 ? fabs(eg[i] * s) : R(0));
+      gl = fmin(gl, dg[i] * s - r);
+      gu = fmax(gu, dg[i] * s + r);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -270,15 +312,23 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
       gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
     }
     const R span = fmax(fabs(gl), fabs(gu));
-    glim[0] = gl - R(4) * rlim<R>::eps() * span - rlim<R>::pivmin();
-    glim[1] = gu + R(4) * rlim<R>::eps() * span + rlim<R>::pivmin();
+    lim[0] = gl - R(4) * rlim<R>::eps() * span - rlim<R>::pivmin();
+    lim[1] = gu + R(4) * rlim<R>::eps() * span + rlim<R>::pivmin();
+    lim[2] = s;
+    lim[3] = unit;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const R e = (i < n - 1) ? eg[i] * lim[2] : R(0);
+    d[i] = dg[i] * lim[2];
+    e2[i] = e * e;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * WARPS + wid;
   if (t >= ell) return;
   const int idx = n - 1 - t;  // ascending index of the t-th largest eigenvalue
-  R lo = glim[0], hi = glim[1];
+  R lo = lim[0], hi = lim[1];
   const R tol = R(2) * rlim<R>::eps() * fmax(fabs(lo), fabs(hi));
   for (int it = 0; it < 64 && hi - lo > tol; ++it) {
     const R x = lo + (hi - lo) * R(lane + 1) / R(33);
@@ -291,7 +341,7 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
     lo = nlo;
     hi = nhi;
   }
-  if (lane == 0) ((R*)P.lam)[t] = R(0.5) * (lo + hi);
+  if (lane == 0) ((R*)P.lam)[t] = R(0.5) * (lo + hi) * lim[3];
 }
 
 // ------------------------------------------------------------------ stage 3
