@@ -6,13 +6,20 @@
 
 // float: the square root and the division by beta come from one reciprocal
 // square root with a Newton step (an IEEE square root and four IEEE divisions in a
-// row are a third of a column's latency); an underflowing norm leaves the
-// column as it is.
+// row are a third of a column's latency).  Near the ends of the range (a column of
+// norm below 1e-18 or above 3e18) the reciprocals leave it, and the square root and
+// divisions are taken; a norm that underflows to zero leaves the column as it is.
 AGB_DEV void reflector(float2 alpha, float xn2, float& beta, float2& t, float2& sc) {
   const float ss = fmaf(alpha.x, alpha.x, fmaf(alpha.y, alpha.y, xn2));
-  if ((xn2 == 0.f && alpha.y == 0.f) || ss <= 1e-36f) {
+  if ((xn2 == 0.f && alpha.y == 0.f) || ss == 0.f) {
     beta = alpha.x;
     t = sc = make_float2(0.f, 0.f);
+    return;
+  }
+  if (!(ss > 1e-36f && ss < 1e37f)) {
+    beta = -copysignf(sqrtf(ss), alpha.x);
+    t = make_float2((beta - alpha.x) / beta, -alpha.y / beta);
+    sc = cinv(make_float2(alpha.x - beta, alpha.y));
     return;
   }
   float y = rsqrtf(ss);
