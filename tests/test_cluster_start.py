@@ -33,17 +33,19 @@ def test_the_cluster_kernels_are_found():
 @pytest.mark.gpu
 def test_one_by_one_matrix_on_a_forced_cluster():
     """A cluster size set for a size class holds for n = 1 too: only the CTA that has the
-    row writes the result."""
+    row writes the result.  Bound (2 n + 24) u of test_tridiag_reg.py (bisection ends
+    within a few u of the diagonal)."""
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA GPU")
     from atlasq_gb300 import _lib, ops
     lib = _lib.load()
     H = torch.arange(1.0, 65.0, dtype=torch.complex128, device="cuda:0").reshape(64, 1, 1)
-    for dtype, code in ((torch.complex64, _lib.AGB_C64), (torch.complex128, _lib.AGB_C128)):
+    for dtype, code, u in ((torch.complex64, _lib.AGB_C64, 2.0 ** -24), (torch.complex128, _lib.AGB_C128, 2.0 ** -53)):
         assert lib.agb_set_tridiag_cluster(code, 24, 64, 8, 512) == 0  # the class of n <= 32, more than 32 matrices
         try:
             w, _ = ops.heevd(H.to(dtype))
         finally:
             assert lib.agb_set_tridiag_cluster(code, 24, 64, 0, 512) == 0
-        assert torch.equal(w.reshape(-1).double(), H.real.reshape(-1))
+        ref = H.real.reshape(-1)
+        assert bool(((w.reshape(-1).double() - ref).abs() <= 26 * u * ref).all())
