@@ -40,7 +40,7 @@ def test_one_by_one_matrix_on_a_forced_cluster():
         pytest.skip("needs a CUDA GPU")
     from atlasq_gb300 import _lib, ops
     lib = _lib.load()
-    H = torch.arange(1.0, 65.0, dtype=torch.complex128, device="cuda:0").reshape(64, 1, 1)
+    H = torch.arange(1.0, 65.0).to(torch.complex128).to("cuda:0").reshape(64, 1, 1)
     for dtype, code, u in ((torch.complex64, _lib.AGB_C64, 2.0 ** -24), (torch.complex128, _lib.AGB_C128, 2.0 ** -53)):
         assert lib.agb_set_tridiag_cluster(code, 24, 64, 8, 512) == 0  # the class of n <= 32, more than 32 matrices
         try:
