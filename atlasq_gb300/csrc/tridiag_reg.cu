@@ -126,7 +126,7 @@ AGB_HD Layout layout(int cpt, int rce) {
   L.part = o;  o += (nc + 256) * 8;
   L.pr = o;    o += nc * 16;
   L.rowsl = o; o += nc * 8;
-  L.dots = o;  o += 32 * 4;
+  L.dots = o;  o += 48 * 4;
   L.red = o;   o += 16 * 4;
   L.bars = o;  o += 32;
   L.f4 = o;    o += (size_t)rce * 16;
@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(NT, 1)
   float2* part = (float2*)(smem + L.part);    // [V][S] partial p of this CTA's column slice
   float2* pr = (float2*)(smem + L.pr);        // [NC][2] p and row j + 1, side by side
   float2* rowsl = (float2*)(smem + L.rowsl);  // [S] row j + 1 over the own slice
-  float* wdots = (float*)(smem + L.dots);     // [16] v^H A v shares of the warps that report here
-  float* dots = wdots + 16;                   // [16] shares of the CTAs
+  float* wdots = (float*)(smem + L.dots);     // [2][16] v^H A v shares of the warps that report here, by step
+  float* dots = wdots + 32;                   // [16] shares of the CTAs
   float* red = (float*)(smem + L.red);        // [NW] norm partials, then alpha at red[8..9] (red[10..11] takes the others' stores)
   const uint32_t bar1 = smem_u32(smem + L.bars), bar2 = bar1 + 8;  // partials; their sums
   volatile int* stop = (volatile int*)(smem + L.bars + 16);
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(NT, 1)
   }
   const int base = nr - RR;  // slot of register row 0 (may be negative)
   const int ngm = (base > 0 ? base : 0) - nsm;
-  const int S = exchange::slice(n, Ce, CPT);  // columns of a CTA's slice
+  const int S = ((n + Ce - 1) / Ce + CPT - 1) / CPT * CPT;  // columns of a CTA's slice
 
   // ---- scale by the largest diagonal magnitude (every CTA reads the diagonal)
   float mx = 0;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(NT, 1)
   for (int i = tid; i < 2 * NC; i += NT) pr[i] = zero;
   for (int i = tid; i < NC + 256; i += NT) part[i] = zero;
   for (int i = tid; i < NC; i += NT) rowsl[i] = zero;
-  if (tid < 32) wdots[tid] = 0.f;
+  if (tid < 48) wdots[tid] = 0.f;
   if (tid == 0) {
     *stop = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1));
@@ -267,11 +267,12 @@ __global__ void __launch_bounds__(NT, 1)
   const uint32_t part_addr = peer_addr(smem_u32(part + (size_t)o * S + (c0 - dq * S)), dq);
   const uint32_t row_addr = peer_addr(smem_u32(rowsl + (c0 - dq * S)), dq);
   const uint32_t part_bar = peer_addr(bar1, dq);
-  // the warp's share of v^H A v, and a zero for a CTA that gets no share
+  // the warp's share of v^H A v
   const int dd = exchange::dot_dest(wid, Ce);
   const uint32_t dot_addr = peer_addr(smem_u32(wdots + q * exchange::dot_pitch(Ce) + wid / Ce), dd);
   const uint32_t dot_bar = peer_addr(bar1, dd);
-  const int dz = exchange::zero_dest(wid, Ce);
+  const int ndot = exchange::dot_words(q, Ce) * Ce;  // words of it that arrive here
+  const int nslice = min(n, q * S + S);               // end of the own slice
   int fac[CPT];   // row-factor entry of row c when this owner holds it, else an unused one
   float2 v[CPT];  // own columns of v (step j-1 until A, then step j)
   float2 w[CPT];  // own columns of w of step j-1
@@ -535,13 +536,17 @@ __global__ void __launch_bounds__(NT, 1)
     sd = warp_sum(sd);
     if (lane == 0) {
       if (Ce == 1) wdots[wid] = sd;
-      else send(dot_addr, dot_bar, sd);
-      if (dz >= 0) send(peer_addr(smem_u32(wdots + q), dz), peer_addr(bar1, dz), 0.f);
+      else send(dot_addr + 64u * (j & 1), dot_bar, sd);
+      if (Ce > NW && wid < exchange::zeros(Ce))
+        send(peer_addr(smem_u32(wdots + 16 * (j & 1) + q), NW + wid), peer_addr(bar1, NW + wid), 0.f);
     }
     // off the exchange's critical path: bytes to expect, the stored reflector, the next row
     if (tid == 0 && Ce > 1) {
-      bar_expect(bar1, (uint32_t)exchange::bytes1(n, Ce, V, CPT, q, j));
-      bar_expect(bar2, (uint32_t)exchange::bytes2(n, Ce, j));
+      // pairs of columns of the own slice still in use (CPT at a time)
+      const int f0 = max(q * S, (j + 1) / CPT * CPT);
+      const int sl = nslice > f0 ? (nslice - f0 + CPT - 1) / CPT : 0;
+      bar_expect(bar1, (uint32_t)(sl * (V + 1) * CPT * 8 + ndot * 4));
+      bar_expect(bar2, (uint32_t)((n - 1 - j) * 16 + Ce * 4));
     }
     if (o == 0 && j - c0 >= 0 && j - c0 < CPT) dg[j] = dj;
     if (turn == q && g == 0) {
@@ -578,15 +583,16 @@ __global__ void __launch_bounds__(NT, 1)
     }
     if (!bar_wait(bar1, j & 1)) ok = false;
     // ---------------- C: reduce the own column slice; p and row j+1 of it to every CTA
-    if (wid == NW - 1) {
+    // (each lane reads the shares for itself: a peer that has its word may write the next
+    // step's, into the other half, before the last lane has read these)
+    if (wid == NW - 1 && lane < Ce) {
       float s = 0.f;
 #pragma unroll
       for (int i = 0; i < 16; i += 4) {
-        const float4 z = *(const float4*)(wdots + i);
+        const float4 z = *(const float4*)(wdots + 16 * (j & 1) + i);
         s += (z.x + z.y) + (z.z + z.w);
       }
-      __syncwarp();  // the first word sent lets a peer write the next step's shares
-      if (lane < Ce) send(peer_addr(smem_u32(dots + q), lane), peer_addr(bar2, lane), s);
+      send(peer_addr(smem_u32(dots + q), lane), peer_addr(bar2, lane), s);
     }
     for (int cl = tid; cl < S; cl += NT) {
       const int c = q * S + cl;
