@@ -2,24 +2,19 @@
 // beta = -sign(Re alpha) ||(alpha, x)||, tau, and sc = 1 / (alpha - beta), the factor
 // of x in v = (1, x sc).
 #pragma once
+#include <float.h>
+
 #include "common.cuh"
 
 // float: the square root and the division by beta come from one reciprocal
 // square root with a Newton step (an IEEE square root and four IEEE divisions in a
-// row are a third of a column's latency).  Near the ends of the range (a column of
-// norm below 1e-18 or above 3e18) the reciprocals leave it, and the square root and
-// divisions are taken; a norm that underflows to zero leaves the column as it is.
+// row are a third of a column's latency).  A subnormal squared norm (the column's
+// below 1.1e-19) leaves the column as it is.
 AGB_DEV void reflector(float2 alpha, float xn2, float& beta, float2& t, float2& sc) {
   const float ss = fmaf(alpha.x, alpha.x, fmaf(alpha.y, alpha.y, xn2));
-  if ((xn2 == 0.f && alpha.y == 0.f) || ss == 0.f) {
+  if ((xn2 == 0.f && alpha.y == 0.f) || ss < FLT_MIN) {
     beta = alpha.x;
     t = sc = make_float2(0.f, 0.f);
-    return;
-  }
-  if (!(ss > 1e-36f && ss < 1e37f)) {
-    beta = -copysignf(sqrtf(ss), alpha.x);
-    t = make_float2((beta - alpha.x) / beta, -alpha.y / beta);
-    sc = cinv(make_float2(alpha.x - beta, alpha.y));
     return;
   }
   float y = rsqrtf(ss);
@@ -41,4 +36,17 @@ AGB_DEV void reflector(double2 alpha, double xn2, double& beta, double2& t, doub
   beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
   t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
   sc = cinv(csub(alpha, make_double2(beta, 0.0)));
+}
+
+// The same where nothing scales the matrix, so that a squared norm may be subnormal:
+// such a column is scaled by 2^50 first.
+AGB_DEV void reflector_unscaled(float2 alpha, float xn2, float& beta, float2& t, float2& sc) {
+  const bool small = fmaf(alpha.x, alpha.x, fmaf(alpha.y, alpha.y, xn2)) < FLT_MIN;
+  const float f = small ? 0x1p50f : 1.f;
+  reflector(make_float2(alpha.x * f, alpha.y * f), xn2 * f * f, beta, t, sc);
+  beta *= small ? 0x1p-50f : 1.f;
+  sc = make_float2(sc.x * f, sc.y * f);
+}
+AGB_DEV void reflector_unscaled(double2 alpha, double xn2, double& beta, double2& t, double2& sc) {
+  reflector(alpha, xn2, beta, t, sc);
 }

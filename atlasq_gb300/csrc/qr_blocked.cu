@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(QBT, 1) qr_blocked_kernel(QrbProb<CX> pr0, Qrb
           alpha.y = __shfl_sync(0xffffffffu, am.y, c & 31);
           CX t, sc;
           Rt beta;
-          reflector(alpha, xn2, beta, t, sc);
+          reflector_unscaled(alpha, xn2, beta, t, sc);
 #pragma unroll
           for (int k = 0; k < NK; ++k) {
             const int r = lane + 32 * k;

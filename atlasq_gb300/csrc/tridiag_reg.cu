@@ -228,7 +228,21 @@ __global__ void __launch_bounds__(NT, 1)
   mx = red[0];
 #pragma unroll
   for (int w = 1; w < NW; ++w) mx = fmaxf(mx, red[w]);
-  if (mx == 0.f) mx = 1.f;
+  if (mx == 0.f) {  // no diagonal to scale by: the largest entry (no Gram matrix comes here)
+    __syncthreads();
+    for (int i = tid; i < n * n; i += NT) {
+      const int r = i / n, c = i - r * n;
+      if (c < r) mx = fmaxf(mx, fmaxf(fabsf(H[(int64_t)r * ld + c].x), fabsf(H[(int64_t)r * ld + c].y)));
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+    if (lane == 0) red[wid] = mx;
+    __syncthreads();
+    mx = red[0];
+#pragma unroll
+    for (int w = 1; w < NW; ++w) mx = fmaxf(mx, red[w]);
+    if (mx == 0.f) mx = 1.f;
+  }
   if (q == 0 && tid == 0) *((float*)P.scale) = mx;
   const float inv = 1.f / mx;
 
