@@ -6,9 +6,17 @@
 
 #include "common.cuh"
 
-// float: the square root and the division by beta come from one reciprocal
-// square root with a Newton step (an IEEE square root and four IEEE divisions in a
-// row are a third of a column's latency).  A subnormal squared norm (the column's
+// a / b from r = 1 / b: the product's residual, exact by FMA, corrects it (Markstein)
+AGB_DEV float quotient(float a, float b, float r) {
+  const float q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+
+// float: the square root and the divisions come from one reciprocal square root, a
+// reciprocal and their Newton steps (an IEEE square root and four IEEE divisions in a
+// row are a third of a column's latency), each result rounded once: ||QR - A|| of a
+// 128 x 64 matrix 3.78 u, 4.18 u without the last corrections, 3.93 u with IEEE
+// operations; they cost 0.4% of a 512 x 256 QR.  A subnormal squared norm (the column's
 // below 1.1e-19) leaves the column as it is.
 AGB_DEV void reflector(float2 alpha, float xn2, float& beta, float2& t, float2& sc) {
   const float ss = fmaf(alpha.x, alpha.x, fmaf(alpha.y, alpha.y, xn2));
@@ -19,13 +27,15 @@ AGB_DEV void reflector(float2 alpha, float xn2, float& beta, float2& t, float2& 
   }
   float y = rsqrtf(ss);
   y = fmaf(0.5f * y, fmaf(-ss * y, y, 1.f), y);
-  const float m = ss * y;
+  float m = ss * y;
+  m = fmaf(0.5f * y, fmaf(-m, m, ss), m);  // the square root, rounded once
+  y = fmaf(y, fmaf(-m, y, 1.f), y);        // its reciprocal
   beta = -copysignf(m, alpha.x);
   const float ib = -copysignf(y, alpha.x);
-  t = make_float2((beta - alpha.x) * ib, -alpha.y * ib);
   const float dx = alpha.x - beta;  // no cancellation: beta has the other sign
-  const float id = __frcp_rn(fmaf(dx, dx, alpha.y * alpha.y));
-  sc = make_float2(dx * id, -alpha.y * id);
+  t = make_float2(quotient(-dx, beta, ib), quotient(-alpha.y, beta, ib));
+  const float den = fmaf(dx, dx, alpha.y * alpha.y), id = __frcp_rn(den);
+  sc = make_float2(quotient(dx, den, id), quotient(-alpha.y, den, id));
 }
 AGB_DEV void reflector(double2 alpha, double xn2, double& beta, double2& t, double2& sc) {
   if (xn2 == 0.0 && alpha.y == 0.0) {
