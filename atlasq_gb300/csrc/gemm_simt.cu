@@ -1,6 +1,6 @@
 // SIMT batched complex GEMM for sm_103a, 256 threads.  complex64: 64 x 64 or
 // 32 x 32 output tiles (launch_simt), for small and ragged shapes.  complex128:
-// 16 x 16 tiles, one output per thread: the FP64 pipe does 2 lanes per clock and SM
+// 16 x 16 tiles, one output per thread (32 x 32 for many whole ones): the FP64 pipe does 2 lanes per clock and SM
 // whatever the tile, so what counts is how many SMs a product spreads over and how
 // little of a ragged tile is padding (a 10-gate layer at chi 48: 189 us over its 19 launches, 2043 us with
 // 64 x 64 tiles, 40 CTAs a launch and a third of their area padding).
@@ -87,21 +87,31 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
     __syncthreads();
     if (k0 + 2 * BK < p.K) fetch(k0 + 2 * BK, xa, xb);
     const int kn = min(BK, p.K - k0);
-    if (T == 1 && kn < BK) {  // no padding products on the FP64 pipe
-      for (int k = 0; k < kn; ++k) cfma(acc[0][0], As[buf][k][ty], Bs[buf][k][tx]);
+    auto product = [&](int k) {
+      CX a[T], b[T];
+#pragma unroll
+      for (int i = 0; i < T; ++i) a[i] = As[buf][k][ty + 16 * i];
+#pragma unroll
+      for (int j = 0; j < T; ++j) b[j] = Bs[buf][k][tx + 16 * j];
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) cfma(acc[i][j], a[i], b[j]);
+    };
+    if (kn == BK) {
+#pragma unroll
+      for (int k = 0; k < BK; ++k) product(k);
     } else {
+      // a last step in eighths of products; on the FP64 pipe none is padding
+      int k = 0;
+#pragma unroll 1
+      for (; k + (T == 1 ? 8 : 1) <= kn; k += 8) {
 #pragma unroll
-      for (int k = 0; k < BK; ++k) {
-        CX a[T], b[T];
-#pragma unroll
-        for (int i = 0; i < T; ++i) a[i] = As[buf][k][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < T; ++j) b[j] = Bs[buf][k][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < T; ++i)
-#pragma unroll
-          for (int j = 0; j < T; ++j) cfma(acc[i][j], a[i], b[j]);
+        for (int u = 0; u < 8; ++u) product(k + u);
       }
+      if (T == 1)
+#pragma unroll 1
+        for (; k < kn; ++k) product(k);
     }
   };
   fetch(0, va[0], vb[0]);
@@ -133,26 +143,36 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmProb* __restri
 
 }  // namespace
 
-// complex64: 64 x 64 tiles (K-step 16) where they give every SM one, else 32 x 32
-// (K-step 32).  32 x 32 tiles are bound by the latency of a step, so it is long, and
-// two are read ahead from addresses formed once: a 256 x 512 x 256 product takes
-// 12.4 us (16.1 with K-step 16; 23 reading one step ahead, 27 with a transposed
-// operand; 32 CTAs of 64 x 64 took 40), five 200 x 400 x 200 27 (30), 64^3 5.2
-// (7.3), 1024^3 on 64 x 64 tiles 221 (248).
+// complex64: 64 x 64 tiles where they give every SM one and pad less than half as much
+// again as 32 x 32 ones (1000 products of 33^3: 37 us, 43 on 32 x 32; 152 of 65^3,
+// three quarters more area: 36 and 27; 4096 of 8^3: 42 and 16).  K-step 8: with 16 the
+// short products (K = 8 to 20) load and add up to a whole step of padding.
+// 32 x 32 tiles: up to two CTAs an SM they are bound by the latency of a step, so it is
+// long (K-step 32), and two are read ahead from addresses formed once: a 256 x 512 x 256
+// product takes 12.4 us (16.1 with K-step 16; 23 reading one step ahead, 27 with a
+// transposed operand; 32 CTAs of 64 x 64 took 40), 1 x 1000 x 1000 43 (K-step 8: 45).
+// Beyond that, and for short K, K-step 8: 20 of 200 x 400 x 200 84 (94), 200 of 32^3
+// 5.2 (5.9), 300 of 8^3 3.4 (4.8).
+// complex128: 32 x 32 tiles (K-step 8) where the bounds are multiples of 32 and there are
+// ten CTAs an SM, so that a last wave costs little: 152 products of 128^3 2136 us
+// (16 x 16: 2190), 1000 of 64 x 64 x 8 315 (343); 160 of 64^3, 640 CTAs, 344 (302).
 template <typename CX>
-static int launch_simt(const GemmProb* probs, const StridedBatch& sb, int count, int64_t M, int64_t N,
+static int launch_simt(const GemmProb* probs, const StridedBatch& sb, int count, int64_t M, int64_t N, int64_t K,
                        cudaStream_t s) {
   auto tiles = [&](int b) { return ((N + b - 1) / b) * ((M + b - 1) / b); };
   int b = 16;
-  if (sizeof(CX) == 8) b = tiles(64) * count >= 152 ? 64 : 32;
+  if (sizeof(CX) == 8) b = tiles(64) * count >= 152 && 8 * tiles(64) < 3 * tiles(32) ? 64 : 32;
+  else if (M % 32 == 0 && N % 32 == 0 && tiles(32) * count >= 1520) b = 32;
   const int64_t t = tiles(b), tn = (N + b - 1) / b;
   if (t > 0x7fffffff) return AGB_ERR_UNSUPPORTED;
   const dim3 grid((unsigned)t, 1, count);
   if constexpr (sizeof(CX) == 16) {
-    gemm_simt_kernel<CX, 16, 16, 1><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    if (b == 32) gemm_simt_kernel<CX, 32, 8, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    else gemm_simt_kernel<CX, 16, 16, 1><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
   } else {
-    if (b == 64) gemm_simt_kernel<CX, 64, 16, 4><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
-    else gemm_simt_kernel<CX, 32, 32, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    if (b == 64) gemm_simt_kernel<CX, 64, 8, 4><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    else if (K > 32 && t * count <= 304) gemm_simt_kernel<CX, 32, 32, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
+    else gemm_simt_kernel<CX, 32, 8, 2><<<grid, 256, 0, s>>>(probs, sb, (int)tn);
   }
   AGB_CHECK_LAUNCH();
   return AGB_OK;
@@ -165,7 +185,7 @@ int launch_gemm_probs(const GemmProb* probs, int count, int maxM, int maxN, cuda
   if (sizeof(CX) == 8 && ctx && ctx->tc_scratch && maxM >= 64 && maxN >= 64 && maxK >= 32 &&
       ctx->tc_bytes >= tc_gemm_scratch_bytes(count, maxM, maxN, maxK))
     return launch_gemm_tc(probs, count, maxM, maxN, maxK, ctx->tc_scratch, ctx->tc_bytes, ctx->status, s);
-  return launch_simt<CX>(probs, StridedBatch{}, count, maxM, maxN, s);
+  return launch_simt<CX>(probs, StridedBatch{}, count, maxM, maxN, maxK, s);
 }
 
 template int launch_gemm_probs<float2>(const GemmProb*, int, int, int, cudaStream_t, const GemmCtx*, int);
@@ -214,6 +234,6 @@ extern "C" int agb_cgemm_batched(int dtype, char opA, char opB, int batch, int M
   sb.sB = strideB;
   sb.sC = strideC;
   cudaStream_t s = (cudaStream_t)stream;
-  return dtype == AGB_C64 ? launch_simt<float2>(nullptr, sb, batch, M, N, s)
-                          : launch_simt<double2>(nullptr, sb, batch, M, N, s);
+  return dtype == AGB_C64 ? launch_simt<float2>(nullptr, sb, batch, M, N, K, s)
+                          : launch_simt<double2>(nullptr, sb, batch, M, N, K, s);
 }

@@ -563,8 +563,8 @@ extern "C" int agb_gemm_list(int dtype, int tensor_cores, const void* probs, int
     return launch_gemm_tc(p, count, maxM, maxN, maxK, status_dev, tc_gemm_scratch_bytes(count, maxM, maxN, maxK),
                           status_dev, s);
   }
-  return dtype == AGB_C64 ? launch_gemm_probs<float2>(p, count, maxM, maxN, s)
-                          : launch_gemm_probs<double2>(p, count, maxM, maxN, s);
+  return dtype == AGB_C64 ? launch_gemm_probs<float2>(p, count, maxM, maxN, s, nullptr, maxK)
+                          : launch_gemm_probs<double2>(p, count, maxM, maxN, s, nullptr, maxK);
 }
 
 // Strided-batch host entry for the tensor-core GEMM (complex64).
