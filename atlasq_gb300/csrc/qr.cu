@@ -172,6 +172,15 @@ AGB_HD QrSmall qr_small_layout(int esz, int M, int N) {
   L.total = L.q + (size_t)kk * L.ld * esz;
   return L;
 }
+// Not for wide matrices: 16 warps take 64 columns at a time, and a round of the
+// FP64 pipe costs the more the more columns wait (us, here and in qr_kernel: 2 x 1024
+// 184 and 49, 16 x 200 445 and 336, 32 x 66 492 and 468, 32 x 60 462 and 462, 4 x 56 39 and
+// 38, 4 x 48 37 and 38, 62 x 62 1273 and 1214, 62 x 56 1071 and 1111); complex64 (1 x 1000
+// 9.7 and 7.9, 4 x 500 19.9 and 19.6, 6 x 500 27.7 and 29.0, 3 x 200 10.7 and 11.1).
+static bool qr_small_pays(int esz, int M, int N) {
+  if (esz == 8) return N <= 256 || M >= 6;
+  return N <= (M >= 8 ? 64 : 48) && !(M >= 60 && N >= 58);
+}
 constexpr int kQrSmallWarps = 16;
 constexpr size_t kQrSmallSmem = 220 * 1024;
 constexpr int kQrSmallCols = 64;  // largest min(M, N) of M N < 64 x 64
@@ -337,7 +346,7 @@ extern "C" int agb_qr(int dtype, const void* A, int M, int N, int transA, void* 
                        : launch_qr_cluster<double2>((const double2*)A, M, N, transA, (double2*)Q, (double2*)R,
                                                     trans_out, (double2*)Qw, s);
     if (rc == AGB_OK) return AGB_OK;
-  } else if (qr_small_layout(esz, M, N).total <= kQrSmallSmem) {
+  } else if (qr_small_pays(esz, M, N) && qr_small_layout(esz, M, N).total <= kQrSmallSmem) {
     const size_t sm = qr_small_layout(esz, M, N).total;
     const int nw = (N + 3) / 4 < kQrSmallWarps ? (N + 3) / 4 : kQrSmallWarps;
     if (dtype == AGB_C64) {
