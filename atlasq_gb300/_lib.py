@@ -27,6 +27,7 @@ AGB_RUN_REPAIR = 1
 AGB_RUN_NO_GUARD = 2
 AGB_RUN_REPAIR_LATER = 4
 AGB_RUN_REPAIR_ONLY = 8
+AGB_REPAIR_WANTED = 4
 
 # descriptor fields (enum agb_desc_field)
 D_A, D_B, D_U, D_CHIL, D_CHIM, D_CHIR, D_CAP, D_EPS = 0, 1, 2, 3, 4, 5, 6, 7

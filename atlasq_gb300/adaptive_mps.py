@@ -30,7 +30,6 @@ from .diagnostics import MPSStatistics
 from .truncation import check_entropy_sanity
 
 _C64, _C128 = torch.complex64, torch.complex128
-_ORTH_GUARD2 = float(np.float32(0.3) * np.float32(0.3))  # kOrthGuard squared (csrc/heevd.cuh)
 
 
 @dataclass
@@ -741,7 +740,7 @@ def _run_pipeline(entries, dt, ells, all_vectors=False, cluster_tol=None, spectr
     # a gate whose eigenvalue-guided eigenvector count fell short is re-run with
     # every vector on the device; AGB_ERR_RANK then only means a predicted ell
     # below the rank, which the caller re-runs at full size.  The results come
-    # back anyway, so the re-run is issued only when some gate needs it.
+    # back anyway, so the re-run is issued only when the device asks for it.
     gflag = 0 if guard else _lib.AGB_RUN_NO_GUARD
 
     def run(flags):
@@ -750,8 +749,7 @@ def _run_pipeline(entries, dt, ells, all_vectors=False, cluster_tol=None, spectr
         return desc_dev.cpu().numpy()
 
     out = run(_lib.AGB_RUN_REPAIR_LATER)
-    overlap = ~(np.ascontiguousarray(out[:, _lib.D_ORTH]).view(np.float64) <= _ORTH_GUARD2)
-    if (out[:, _lib.D_STATUS] == _lib.AGB_ERR_RANK).any() or (guard and (overlap & (out[:, _lib.D_MODE] == 0)).any()):
+    if (out[:, _lib.D_REPAIR] == _lib.AGB_REPAIR_WANTED).any():
         out = run(_lib.AGB_RUN_REPAIR_ONLY)
     sig = None
     if spectra:

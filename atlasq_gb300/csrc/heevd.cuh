@@ -76,7 +76,7 @@ struct HeevdProb {
   double ctol;       // cluster tolerance relative to max|lambda| (kClusterTol unless repaired)
   void* band;        // scratch of the two-stage tridiagonalisation (block-reflector factors,
                      // exchange rows, band-stage reflectors), tridiag_2stage.cu
-  int fail;          // set when a bounded wait of the band stage expired
+  int fail;          // set when a bounded wait of the tridiagonalisation expired
 };
 
 // Bytes of the two-stage scratch for an n x n problem (the larger of the band

@@ -407,13 +407,10 @@ __global__ void __launch_bounds__(kSmallThreads) small_gate_kernel(int64_t* __re
       status = AGB_ERR_NOCONV;
       k = 0;
     }
-    // repair: every vector where the eigenvalue-guided count fell short, the wide
-    // cluster tolerance where two vectors converged onto one
-    const bool overlap = guard && orth_exceeds(omax) && mode0 == 0 && (status == AGB_OK || status == AGB_ERR_RANK);
-    const bool short_count = status == AGB_ERR_RANK && nv < ell && mode0 == 0;
-    if (attempt == 0 && repair && (overlap || short_count)) {
-      repaired = (short_count ? 1 : 0) | (overlap ? 2 : 0);
-      if (overlap) ctol = kClusterTolWide;
+    const int bits = repair_bits(status, nv, ell, mode0, omax, guard);
+    if (attempt == 0 && repair && bits) {
+      repaired = bits;
+      if (bits & 2) ctol = kClusterTolWide;
       nv = ell;
       __syncthreads();
       continue;

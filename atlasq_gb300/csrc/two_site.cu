@@ -558,6 +558,16 @@ __global__ void __launch_bounds__(256) norms_kernel(const int64_t* __restrict__ 
   }
 }
 
+// What a repair pass would do for a gate (AGB_D_REPAIR bits): every vector where the
+// eigenvalue-guided count fell short, the wide cluster tolerance where two vectors
+// converged onto one.
+AGB_DEV int repair_bits(int64_t status, int nvec, int ell, int64_t mode, unsigned orth_max2, int guard) {
+  if (mode != 0) return 0;
+  const bool short_count = status == AGB_ERR_RANK && nvec < ell;
+  const bool overlap = guard && orth_exceeds(orth_max2) && (status == AGB_OK || status == AGB_ERR_RANK);
+  return (short_count ? 1 : 0) | (overlap ? 2 : 0);
+}
+
 // One block per gate.  sigma_t^2 = ||AV[:, t]||^2, sorted descending; then the
 // reference rank rule with torch-CPU float32 semantics for complex64:
 //   E = cumsum(S*S) accumulated in double, each partial rounded to float32;
@@ -670,6 +680,8 @@ __global__ void __launch_bounds__(1024) rank_kernel(int64_t* __restrict__ desc, 
     status = (int)D[AGB_D_STATUS];
     k = 0;
   }
+  if (pass == 0 && repair_bits(status, hp[g].nvec, ell, mode0, hp[g].orth_max2, guard))
+    D[AGB_D_REPAIR] = AGB_REPAIR_WANTED;  // until the repair pass says what it did
   D[AGB_D_K] = k;
   D[AGB_D_EPSLOC] = bitsd(eps_local);
   D[AGB_D_ENTROPY] = bitsd(entropy);
@@ -765,19 +777,16 @@ __global__ void repair_setup_kernel(int64_t* __restrict__ desc, int ng, char* ws
   HeevdProb* hp = (HeevdProb*)ws;
   GemmProb* gp = (GemmProb*)(ws + agb_align((size_t)ng * sizeof(HeevdProb)));
   const int ell = (int)D[AGB_D_ELL];
-  const int st = (int)D[AGB_D_STATUS];
-  const bool short_count = st == AGB_ERR_RANK && hp[g].nvec < ell && D[AGB_D_MODE] == 0;
-  const bool overlap =
-      guard && orth_exceeds(hp[g].orth_max2) && D[AGB_D_MODE] == 0 && (st == AGB_OK || st == AGB_ERR_RANK);
-  if (short_count || overlap) {
+  const int bits = repair_bits(D[AGB_D_STATUS], hp[g].nvec, ell, D[AGB_D_MODE], hp[g].orth_max2, guard);
+  if (bits) {
     hp[g].redo = 1;
     hp[g].nvec = ell;
     hp[g].skip_vectors = 0;
-    if (overlap) hp[g].ctol = kClusterTolWide;
+    if (bits & 2) hp[g].ctol = kClusterTolWide;
     gp[3 * ng + g].N = ell;
     gp[3 * ng + g].M = 2 * (int)D[AGB_D_CHIL];
     D[AGB_D_STATUS] = AGB_OK;
-    D[AGB_D_REPAIR] = (short_count ? 1 : 0) | (overlap ? 2 : 0);
+    D[AGB_D_REPAIR] = bits;
   } else {
     hp[g].redo = 0;
     hp[g].skip_vectors = 1;

@@ -88,7 +88,9 @@ enum agb_desc_field {
                        *       keep (from the eigenvalues, plus a pad); -1: all ell */
   AGB_D_REPAIR = 31,  /* (out) vector phase re-run on the device: bit 0 the guided
                        *       count fell short, bit 1 the eigenvectors failed the
-                       *       orthogonality guard (re-run with tolerance 1e-2)   */
+                       *       orthogonality guard (re-run with tolerance 1e-2);
+                       *       AGB_REPAIR_WANTED (bit 2, alone): left to the second
+                       *       call of AGB_RUN_REPAIR_LATER                       */
   AGB_D_NFIELDS = 32
 };
 
@@ -126,8 +128,8 @@ int agb_two_site_plan(int dtype, int ngates, int64_t* desc_host, size_t* ws_byte
                             * neither repair nor reject on it */
 #define AGB_RUN_REPAIR_LATER 4 /* flags: leave those gates to a second call (below); a caller
                                 * that reads the results back anyway issues it only when some
-                                * gate reports AGB_ERR_RANK or an AGB_D_ORTH (AGB_D_MODE 0) above
-                                * 0.3 squared */
+                                * gate reports AGB_REPAIR_WANTED */
+#define AGB_REPAIR_WANTED 4 /* value of AGB_D_REPAIR after AGB_RUN_REPAIR_LATER */
 #define AGB_RUN_REPAIR_ONLY 8 /* flags: that second call, on the same descriptors and workspace */
 int agb_two_site_run(int dtype, int ngates, const int64_t* desc_dev, int64_t* desc_dev_out,
                      int max_chiL, int max_chiM, int max_chiR, int max_ell, void* ws, size_t ws_bytes,
