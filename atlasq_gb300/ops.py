@@ -217,6 +217,11 @@ class ProductList:
         return len(self.groups) - 1
 
     def upload(self):
+        self.stream = stream_ptr(self.device)
+        self.status = ptr(_tc_status_word(self.device))
+        if torch.cuda.is_current_stream_capturing():  # no copy of host memory there: product by product
+            self.dev = None
+            return self
         assert _lib.load().agb_gemm_prob_bytes() == _PROB.itemsize
         arr = np.zeros(len(self.rows), dtype=_PROB)
         if self.rows:
@@ -226,15 +231,26 @@ class ProductList:
                 arr[name] = num[:, k]
             arr["C"], arr["ldc"], arr["alpha_re"] = arr["D"], arr["ldd"], 1.0
         self.dev = torch.from_numpy(arr.view(np.uint8)).to(self.device)
-        self.base, self.stream = self.dev.data_ptr(), stream_ptr(self.device)
-        self.status = ptr(_tc_status_word(self.device))
+        self.base = self.dev.data_ptr()
         return self
 
     def launch(self, g):
         lib = _lib.load()
         for on, first, count, M, N, K in self.groups[g]:
+            if self.dev is None:
+                for p in self.rows[first:first + count]:
+                    self._launch_one(lib, on, *p)
+                continue
             check(lib.agb_gemm_list(self.code, on, self.base + first * _PROB.itemsize, count, M, N, K, self.status,
                                     self.stream), "gemm_list")
+
+    def _launch_one(self, lib, on, M, N, K, opA, opB, A, lda, B, ldb, D, ldd):
+        args = (opA.encode(), opB.encode(), 1, M, N, K, A, lda, 0, B, ldb, 0, D, ldd, 0, 1.0, 0.0, 0.0, 0.0)
+        if on:
+            ws = workspace(lib.agb_cgemm_tc_workspace(1, M, N, K), self.device, "gemm_tc")
+            check(lib.agb_cgemm_tc_async(*args, ptr(ws), ws.numel(), self.status, self.stream), "cgemm_tc")
+        else:
+            check(lib.agb_cgemm_batched(self.code, *args, self.stream), "cgemm")
 
 
 _TC_STATUS = {}
