@@ -198,19 +198,24 @@ __global__ void __launch_bounds__(1024) tridiag_kernel(const HeevdProb* __restri
 // the recurrence see the same sign.
 // Range: the caller scales T so that the largest |d_i|, |e_i| is in [1, 4).  A step then
 // grows the pair (p_i, p_{i-1}) by at most 2^5, and it is rescaled by a power of two every
-// U steps.  It may shrink by any factor (d_i - x and e_i both small): where the U steps
-// took it below `low`, they are repeated with a rescaling each.  In a pair that stayed above,
-// an underflow changes d_i or e_i by less than 2^-32 (float; 2^-300 double).
+// U steps.  It may shrink by any factor (d_i - x and e_i both small): where U steps took
+// it below `low`, the count is repeated with a rescaling in every step.  In a pair that
+// stayed above, an underflow changes d_i by less than 2^-28 (float; p_i is then below 2^-126 and
+// off by 2^-150, and p_{i-1} at least low / 2^15; 2^-139 double), a tenth of the rounding of x.
+// That takes |d_i - x| and e_i^2 below 2^-26 several times in a row, so the repetition is rare.
+// One test a count: testing and repeating group by group cost 40% (256 columns 29 -> 40 us).
 AGB_DEV unsigned sign_bits(float a, float b) { return (unsigned)(__float_as_int(a) ^ __float_as_int(b)) >> 31; }
 AGB_DEV unsigned sign_bits(double a, double b) { return (unsigned)(__double2hiint(a) ^ __double2hiint(b)) >> 31; }
-// 2^-exponent of the larger of a and b, which is below 2^126 (2^1022)
-AGB_DEV float pair_scale(float a, float b) {
-  const int h = max(__float_as_int(a) & 0x7f800000, __float_as_int(b) & 0x7f800000);
-  return __int_as_float(0x7f000000 - h);
+// Exponent bits of the larger of a and b, and 2^-exponent for them (exponents below 2^126, 2^1022).
+AGB_DEV int pair_exp(float a, float b) {
+  return max(__float_as_int(a) & 0x7f800000, __float_as_int(b) & 0x7f800000);
 }
-AGB_DEV double pair_scale(double a, double b) {
-  const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
-  return __hiloint2double(0x7fe00000 - h, 0);
+AGB_DEV int pair_exp(double a, double b) {
+  return max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
+}
+template <typename R> AGB_DEV R exp_inverse(int h) {
+  if constexpr (sizeof(R) == 4) return __int_as_float(0x7f000000 - h);
+  else return __hiloint2double(0x7fe00000 - h, 0);
 }
 // 2^e with 2^e <= a < 2^(e+1) (e kept where 2^-e is a normal number too), and 2^-e
 AGB_DEV void power_of(float a, float& p, float& inv) {
@@ -227,9 +232,10 @@ template <typename R>
 AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
   constexpr int U = sizeof(R) == 8 ? 8 : 4;
   constexpr R tiny = sizeof(R) == 8 ? R(0x1p-200) : R(0x1p-60f);
-  constexpr R low = sizeof(R) == 8 ? R(0x1p-400) : R(0x1p-60f);
+  constexpr int low = sizeof(R) == 8 ? (1023 - 900) << 20 : (127 - 106) << 23;  // exponent bits
   R p2 = 1, p1 = d[0] - x;
   if (p1 == R(0)) p1 = -tiny;
+  const R first = p1;
   int cnt = p1 < R(0);
   auto step = [&](int i) {
     R p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
@@ -238,13 +244,27 @@ AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
     p2 = p1;
     p1 = p;
   };
-  auto rescale = [&]() {
-    const R f = pair_scale(p1, p2);
+  auto rescale = [&](int h) {
+    const R f = exp_inverse<R>(h);
     p1 *= f;
     p2 *= f;
   };
-  auto sure_step = [&](int i) {
-    rescale();
+  int i = 1, least = pair_exp(p1, p2);
+  for (; i + U <= n; i += U) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) step(i + k);
+    const int h = pair_exp(p1, p2);
+    least = min(least, h);
+    rescale(h);
+  }
+  for (; i < n; ++i) step(i);
+  if (min(least, pair_exp(p1, p2)) >= low) return cnt;
+  p2 = 1;
+  p1 = first;
+  cnt = p1 < R(0);
+#pragma unroll 1
+  for (i = 1; i < n; ++i) {
+    rescale(pair_exp(p1, p2));
     const R p = fma(d[i] - x, p1, -(e2[i - 1] * p2));
     if (p == R(0)) {
       ++cnt;
@@ -255,31 +275,14 @@ AGB_DEV int sturm_count(const R* d, const R* e2, int n, R x) {
       p2 = p1;
       p1 = p;
     }
-  };
-  int i = 1;
-  for (; i + U <= n; i += U) {
-    const R b1 = p1, b2 = p2;
-    const int before = cnt;
-#pragma unroll
-    for (int k = 0; k < U; ++k) step(i + k);
-    if (!(fmax(fabs(p1), fabs(p2)) >= low)) {
-      p1 = b1;
-      p2 = b2;
-      cnt = before;
-#pragma unroll 1
-      for (int k = 0; k < U; ++k) sure_step(i + k);
-    }
-    rescale();
   }
-#pragma unroll 1
-  for (; i < n; ++i) sure_step(i);
   return cnt;
 }
 
 // A warp per eigenvalue, WARPS of them per CTA: 8 for float; 2 for double, whose
-// steps share the FP64 pipe of the SM (10 problems of n = 96: 215 us, 499 with a
-// division a step, 918 on a quarter of the CTAs).  float, with and without the
-// division: one problem of n = 1024 259 and 96 us, 20 of n = 512 199 and 105.
+// steps share the FP64 pipe of the SM (10 problems of n = 96: 234 us, 499 with a
+// division a step, 918 on a quarter of the CTAs).  float: half the eigenvalues of one
+// problem of n = 1024 105 us (259 with a division a step), of 20 of n = 512 170.
 template <typename R, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __restrict__ probs) {
   const HeevdProb P = probs[blockIdx.y];
@@ -288,47 +291,58 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* d = (R*)smem_raw;
   R* e2 = d + n;
-  __shared__ R lim[4];  // Gershgorin interval of the scaled T; the scale and its inverse
+  __shared__ R lim[3][WARPS];  // per warp: largest |d|, |e|; ends of the Gershgorin interval
   const R* dg = (const R*)P.d;
   const R* eg = (const R*)P.e;
-  if (threadIdx.x < 32) {
-    // min and max do not depend on the order
-    R big = 0;
-    for (int i = threadIdx.x; i < n; i += 32)
-      big = fmax(big, fmax(fabs(dg[i]), i < n - 1 ? fabs(eg[i]) : R(0)));
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // max and min do not depend on the order
+  R big = 0;
+  for (int i = threadIdx.x; i < n; i += 32 * WARPS) {
+    const R di = dg[i], ei = (i < n - 1) ? eg[i] : R(0);
+    d[i] = di;
+    e2[i] = ei;
+    big = fmax(big, fmax(fabs(di), fabs(ei)));
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
-    R unit, s;
-    power_of(big, unit, s);
-    R gl = dg[0] * s, gu = gl;
-    for (int i = threadIdx.x; i < n; i += 32) {
-      const R r = (i > 0 ? fabs(eg[i - 1] * s) : R(0)) + (i < n - 1 ? fabs(eg[i] * s) : R(0));
-      gl = fmin(gl, dg[i] * s - r);
-      gu = fmax(gu, dg[i] * s + r);
-    }
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) lim[0][wid] = big;
+  __syncthreads();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
-      gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
-    }
-    const R span = fmax(fabs(gl), fabs(gu));
-    lim[0] = gl - R(4) * rlim<R>::eps() * span - rlim<R>::pivmin();
-    lim[1] = gu + R(4) * rlim<R>::eps() * span + rlim<R>::pivmin();
-    lim[2] = s;
-    lim[3] = unit;
+  for (int w = 0; w < WARPS; ++w) big = fmax(big, lim[0][w]);
+  R unit, s;  // T is scaled by s = 1 / unit
+  power_of(big, unit, s);
+  R gl = d[0] * s, gu = gl;
+  for (int i = threadIdx.x; i < n; i += 32 * WARPS) {
+    const R di = d[i] * s, r = (i > 0 ? fabs(e2[i - 1] * s) : R(0)) + fabs(e2[i] * s);
+    gl = fmin(gl, di - r);
+    gu = fmax(gu, di + r);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
+    gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
+  }
+  if (lane == 0) {
+    lim[1][wid] = gl;
+    lim[2][wid] = gu;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const R e = (i < n - 1) ? eg[i] * lim[2] : R(0);
-    d[i] = dg[i] * lim[2];
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    gl = fmin(gl, lim[1][w]);
+    gu = fmax(gu, lim[2][w]);
+  }
+  for (int i = threadIdx.x; i < n; i += 32 * WARPS) {
+    const R e = e2[i] * s;
+    d[i] *= s;
     e2[i] = e * e;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int t = blockIdx.x * WARPS + wid;
   if (t >= ell) return;
   const int idx = n - 1 - t;  // ascending index of the t-th largest eigenvalue
-  R lo = lim[0], hi = lim[1];
+  const R span = fmax(fabs(gl), fabs(gu)), pad = R(4) * rlim<R>::eps() * span;
+  R lo = gl - pad - rlim<R>::pivmin(), hi = gu + pad + rlim<R>::pivmin();
   const R tol = R(2) * rlim<R>::eps() * fmax(fabs(lo), fabs(hi));
   for (int it = 0; it < 64 && hi - lo > tol; ++it) {
     const R x = lo + (hi - lo) * R(lane + 1) / R(33);
@@ -341,7 +355,7 @@ __global__ void __launch_bounds__(32 * WARPS) bisect_kernel(const HeevdProb* __r
     lo = nlo;
     hi = nhi;
   }
-  if (lane == 0) ((R*)P.lam)[t] = R(0.5) * (lo + hi) * lim[3];
+  if (lane == 0) ((R*)P.lam)[t] = R(0.5) * (lo + hi) * unit;
 }
 
 // ------------------------------------------------------------------ stage 3
