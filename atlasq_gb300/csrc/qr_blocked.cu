@@ -32,7 +32,7 @@
 // Inside a panel 15 warps issue ~15 instructions a row for product and update of
 // each column (1400 of its 2800 cycles; the reflector 1200): the reflector is read
 // once, into registers, and in complex64 up to 512 rows padded with zeros to the
-// registers' rows, so that no access is predicated.  512 x 256 on 16 CTAs: 0.57 ms
+// registers' rows, so that no access is predicated.  512 x 256 on 16 CTAs: 0.58 ms
 // (0.65 with predicated reads, twice a column); updates 8 us, the thin Q 6 us a
 // panel.
 #include <cooperative_groups.h>
@@ -622,7 +622,7 @@ static int qr_pair(const int64_t* probs, void* ws, size_t ws_bytes, cudaStream_t
 
 // Two factorisations in one launch where both take the blocked kernel with the
 // same cluster size, one after the other otherwise.  512 x 256, then its mirror image:
-// 1146 us one after the other, 573 us side by side (a chain of 40 sites at chi 256 to
+// 1164 us one after the other, 582 us side by side (a chain of 40 sites at chi 256 to
 // its mixed form: 16.9 -> 9.8 ms at 657 us each).
 extern "C" int agb_qr_pair(int dtype, const int64_t* probs, void* ws, size_t ws_bytes, void* stream) {
   if (dtype != AGB_C64 && dtype != AGB_C128) return AGB_ERR_ARG;

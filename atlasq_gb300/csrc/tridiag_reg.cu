@@ -677,7 +677,7 @@ cudaLaunchConfig_t config(int grid, int C, size_t smem, cudaLaunchAttribute* att
 int launch_tridiag_reg(const HeevdProb* probs, int count, int maxn, int C, cudaStream_t s) {
   if (C < 1 || C > 16 || maxn > 1024) return AGB_ERR_UNSUPPORTED;
   const Form f = form_for(maxn);
-  const int C256 = 8 * count <= 152 ? 8 : 4;  // 0.57 ms on 4 SMs or 0.4x ms on 8 (n = 256)
+  const int C256 = 8 * count <= 152 ? 8 : 4;  // 0.62 ms on 4 SMs or 0.54 on 8 (n = 256)
   const int rce = rowc_entries(maxn, C, C256);
   const size_t off = layout(f.cpt, rce).rows;
   if (off > kRegSmem) return AGB_ERR_UNSUPPORTED;
@@ -728,11 +728,14 @@ int tridiag_reg_clusters(int maxn, int C) {
 
 // CTAs per matrix for `count` matrices of up to maxn columns.  Up to 128 columns
 // are one CTA's registers; up to 256 columns take 8 CTAs while every matrix
-// gets its own SMs (0.51 against 0.58 ms at n = 256) and 4 beyond that.
-// Between 256 and 512 the fewest waves decide: a matrix of n = 512 takes 1.17,
-// 1.32 and 1.42 ms on 16, 10 and 8 CTAs (0.72 + 5.6 / C ms), and a cluster
-// needs its SMs in one GPC.  Above 512 rows spill to L2 below 16 CTAs
-// (n = 1024: 6.4 against 13.7 ms on 8).
+// gets its own SMs (0.54 against 0.62 ms at n = 256) and 4 beyond that.
+// Between 256 and 512 the fewest waves decide: a matrix of n = 512 takes 1.27,
+// 1.40 and 1.52 ms on 16, 10 and 8 CTAs (counted as 0.72 + 5.6 / C), and a cluster
+// needs its SMs in one GPC.  The rule knows the count and the largest n only: 20
+// equal matrices of 512 take 2.80 ms on 10 CTAs and would take 1.80 on 6, but a
+// chain's layer of 20 gates, whose end gates are small, runs all its full-size
+// ones at once on 10 (1.6 ms; 6% more on 6).  Above 512 rows spill to L2 below 16 CTAs
+// (n = 1024: 6.8 against 14.4 ms on 8).
 int tridiag_reg_ctas(int maxn, int count) {
   if (maxn <= 128) return 1;
   if (maxn <= 256) return 8 * count <= 152 ? 8 : 4;

@@ -589,12 +589,12 @@ def main():
                              "frac": (wf / t_dom / 1e12) / fp32_peak if t_dom > 0 else 0.0}
         # DRAM bytes of ONE launch (one saturated layer: 20 Gram matrices of
         # 512 x 512) from an ncu capture of this kernel on 20 matrices of that
-        # size: read 21 728 768 B, written 0 B, against that launch's 20 x 2 n^2 x
+        # size: read 21 733 120 B, written 0 B, against that launch's 20 x 2 n^2 x
         # 8 B = 83 886 080 algorithmic bytes (the rest is served from L2, where the
         # Gram GEMM left it).  Per launch, not per step.
-        roof["traffic"] = 21728768
+        roof["traffic"] = 21733120
         roof["traffic_per_launch"] = {"matrices": 20, "n": 512, "algorithmic_bytes": 20 * 2 * 512 * 512 * 8,
-                                      "dram_bytes": 21728768,
+                                      "dram_bytes": 21733120,
                                       "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch"}
 
     line = {"metric": METRIC, "value": value, "unit": "gates/s", "n_gpus": ws, "steps": args.steps,
