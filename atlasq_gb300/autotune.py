@@ -46,7 +46,7 @@ def tune_tridiag(n: int, count: int, dtype=torch.complex64, device="cuda"):
     ws = torch.empty(need, dtype=torch.uint8, device=dev)
     bc = ctypes.c_int(0)
     bms = ctypes.c_float(0)
-    # (the library also tries 256 and 512 threads per CTA and keeps the faster)
+    # (complex128: the library also tries 256 and 512 threads per CTA and keeps the faster)
     check(lib.agb_tune_tridiag(code, n_t, count_t, ptr(ws), need, stream_ptr(dev), ctypes.byref(bc),
                                ctypes.byref(bms)), "tune_tridiag")
     _done[key] = (bc.value, bms.value)
